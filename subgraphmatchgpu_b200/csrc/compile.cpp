@@ -532,6 +532,19 @@ static void RequireSiblingLayout(Program& p) {
   }
 }
 
+// Counts with a kernel of their own, under every plan (the number does not
+// depend on it), while the options ask for nothing about how the steps run: an
+// explicit launch shape, lists without bitmaps, a plan variant or external
+// mode keep the level program.  The root of the task must be pattern vertex 0.
+static CountForm FormOf(const sme_opts& o, const Query& q, const Program& p, bool enumerate) {
+  if (enumerate || !q.enable_ordering || o.execute_mode != SME_IN_MEMORY_GPU || o.warp_granularity != 0 ||
+      o.list_only || o.no_set_reuse || o.reuse_autogen >= 0 || o.compress_level != SME_COMPRESS_SPECIAL ||
+      p.steps[0].kind != S_INIT || p.out_slot[p.steps[0].u] != 0)
+    return C_STEPS;
+  if (q.type == 1) return C_CYCLE4;
+  return C_STEPS;
+}
+
 Program Compile(const sme_opts& o, bool enumerate, bool loop_free) {
   Query q(o.query_type, o.enable_ordering != 0);
   Program p;
@@ -558,6 +571,7 @@ Program Compile(const sme_opts& o, bool enumerate, bool loop_free) {
   PruneImpliedExclusions(p, loop_free);
   RequireSiblingLayout(p);
   if (!enumerate) AliasRepeatedComputes(p);
+  p.form = FormOf(o, q, p, enumerate);
   for (auto& s : p.steps) {
     std::ostringstream os;
     os << KindName(s.kind) << "(" << (int)s.u << ")";

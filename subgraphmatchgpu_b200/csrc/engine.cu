@@ -21,6 +21,7 @@
 #include <cstdio>
 #include <string>
 
+#include "cycle.cuh"
 #include "engine.h"
 #include "kernels.cuh"
 
@@ -1818,6 +1819,25 @@ uint64_t UploadPackedPipelined(const HostGraph& g, const PackedLists& pk, Device
 }
 }  // namespace
 
+namespace {
+DGraph ViewOf(const DeviceGraph& g) {
+  if (g.hub_slot)
+    return DGraph{g.row_ptrs, g.cols, g.hub_slot, g.bitmaps, g.words, nullptr, g.coarse, g.cwords};
+  return DGraph{g.row_ptrs, g.cols, nullptr, nullptr, 0, nullptr, nullptr, 0};
+}
+
+// Queues k_check_simple on `st` (`flag` cleared by the caller).
+void LaunchCheck(const DeviceGraph& g, bool sym, uint32_t* flag, cudaStream_t st) {
+  if (!g.m) return;
+  const unsigned grid =
+      (unsigned)std::min<uint64_t>((g.m + (uint64_t)kCheckChunk * 8 - 1) / ((uint64_t)kCheckChunk * 8), 148 * 8);
+  if (sym)
+    k_check_simple<true><<<grid, WARP_BLOCK, 0, st>>>(ViewOf(g), (uint32_t)g.n, g.m, flag);
+  else
+    k_check_simple<false><<<grid, WARP_BLOCK, 0, st>>>(ViewOf(g), (uint32_t)g.n, g.m, flag);
+}
+}  // namespace
+
 DeviceGraph* UploadGraph(const HostGraph& g, int device, cudaStream_t stream, uint64_t* h2d) {
   CK(cudaSetDevice(device));
   auto* d = new DeviceGraph();
@@ -1828,7 +1848,8 @@ DeviceGraph* UploadGraph(const HostGraph& g, int device, cudaStream_t stream, ui
   std::shared_ptr<const PackedLists> pk = g.packed;
   uint8_t* scratch = nullptr;
   try {
-    CK(cudaMalloc((void**)&d->row_ptrs, (g.n + 1) * sizeof(uintE)));
+    // one word after the row pointers for k_check_simple's flag
+    CK(cudaMalloc((void**)&d->row_ptrs, (g.n + 2) * sizeof(uintE)));
     CK(cudaMalloc((void**)&d->cols, std::max<uint64_t>(g.m, 1) * sizeof(uintV)));
     if (pk) {
       CheckPacked(g, *pk);
@@ -1857,6 +1878,14 @@ DeviceGraph* UploadGraph(const HostGraph& g, int device, cudaStream_t stream, ui
     size_t fr = 0, tot = 0;
     CK(cudaMemGetInfo(&fr, &tot));
     bytes += BuildHubBitmaps(d, g, stream, dev_alloc, true, fr);
+    uint32_t* flag = reinterpret_cast<uint32_t*>(d->row_ptrs + g.n + 1);
+    CK(cudaMemsetAsync(flag, 0, sizeof(uint32_t), stream));
+    LaunchCheck(*d, true, flag, stream);
+    uint32_t defects = 0;
+    CK(cudaMemcpyAsync(&defects, flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
+    CK(cudaStreamSynchronize(stream));
+    CK(cudaGetLastError());
+    d->defects = (int)defects;
   } catch (...) {
     if (scratch) cudaFree(scratch);
     FreeDeviceGraph(d);
@@ -1957,6 +1986,9 @@ DStep ToDStep(const Step& s) {
   return d;
 }
 
+// Free arena below which every count runs its level program.
+constexpr uint64_t kFormArena = 64ULL << 20;
+
 class Executor {
  public:
   Executor(const Program& prog, const DeviceGraph& g, DeviceContext& ctx, uint32_t* d_out, uint64_t cap)
@@ -2005,7 +2037,7 @@ class Executor {
       F.P = P;
       F.inst[s0.u] = col;
       ++batches_;
-      Level(1, F);
+      if (!CountByForm(col, P)) Level(1, F);
       A_.Release(m);
     }
     CK(cudaEventRecord(ev1, st_));
@@ -2068,16 +2100,66 @@ class Executor {
   uint32_t* ext_cache_ = nullptr;    // device list cache
   uint64_t ext_cap_ = 0, ext_used_ = 0, ext_restarts_ = 0;
 
-  // Loads, for the paths of Fb, the adjacency lists step `ds` intersects into
-  // a device subgraph allocated in the current arena frame (it stays valid
-  // while deeper levels use candidate sets that point into it).
   // The resident graph with its hub bitmaps (`use_bitmaps_` false: lists only).
   DGraph Resident() const {
-    if (use_bitmaps_ && g_.hub_slot)
-      return DGraph{g_.row_ptrs, g_.cols, g_.hub_slot, g_.bitmaps, g_.words, nullptr, g_.coarse, g_.cwords};
+    if (use_bitmaps_) return ViewOf(g_);
     return DGraph{g_.row_ptrs, g_.cols, nullptr, nullptr, 0, nullptr, nullptr, 0};
   }
 
+  // k_check_simple's verdict on the graph (found at upload for a resident
+  // one, else here).
+  uint32_t Defects(bool sym) {
+    if (g_.defects >= 0) return (uint32_t)g_.defects;
+    const size_t mark = A_.Mark();
+    uint32_t* flag = (uint32_t*)A_.Alloc(sizeof(uint32_t));
+    CK(cudaMemsetAsync(flag, 0, sizeof(uint32_t), st_));
+    LaunchCheck(g_, sym, flag, st_);
+    Launched();
+    const uint32_t r = (uint32_t)ReadU32(flag);
+    A_.Release(mark);
+    return r;
+  }
+
+  // Counts the roots col[0..P) with the program's own kernel when it has one
+  // and the graph and the arena allow it; false: run the steps.  Below
+  // kFormArena of free arena the steps' batches stay in charge, whose budget
+  // a caller has set.
+  bool CountByForm(const uint32_t* col, uint32_t P) {
+    if (prog_.form == C_STEPS || ext_cols_ || g_.n > 0xFFFFFFFEu || A_.Free() < kFormArena + (uint64_t)P * 8)
+      return false;
+    if (prog_.form == C_CYCLE4) {
+      if (Defects(true)) return false;
+      CountCycles(col, P);
+      return true;
+    }
+    return false;
+  }
+
+  void CountCycles(const uint32_t* col, uint32_t P) {
+    static std::atomic<bool> set[64];  // per device, once (twice is harmless)
+    const int dv = ctx_.device;
+    if (dv < 0 || dv >= 64 || !set[dv].load(std::memory_order_acquire)) {
+      CK(cudaFuncSetAttribute(k_cycle4_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCycleWarpSmem));
+      CK(cudaFuncSetAttribute(k_cycle4_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCycleCtaSmem));
+      if (dv >= 0 && dv < 64) set[dv].store(true, std::memory_order_release);
+    }
+    uint32_t* ctl = (uint32_t*)A_.Alloc(4 * sizeof(uint32_t));  // next root, queued roots, next queued
+    uint32_t* queue = (uint32_t*)A_.Alloc((size_t)P * 4);
+    const DGraph G = ViewOf(g_);
+    paths_ += P;
+    Timed t = TimerStart();
+    CK(cudaMemsetAsync(ctl, 0, 4 * sizeof(uint32_t), st_));
+    const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sms_ * 2, (P + CYW_WARPS - 1) / CYW_WARPS);
+    k_cycle4_warp<<<grid, CYW_THREADS, kCycleWarpSmem, st_>>>(G, col, P, ctl, queue, ctl + 1, ctrl_);
+    k_cycle4_cta<<<(unsigned)std::min<uint64_t>(sms_, P), CYC_THREADS, kCycleCtaSmem, st_>>>(
+        G, (uint32_t)g_.n, col, queue, ctl + 1, ctl + 2, ctrl_);
+    TimerStop(t, kPhaseComputeCount);
+    launches_ += 2;
+  }
+
+  // Loads, for the paths of Fb, the adjacency lists step `ds` intersects into
+  // a device subgraph allocated in the current arena frame (it stays valid
+  // while deeper levels use candidate sets that point into it).
   DGraph LoadSubgraph(const DFront& Fb, const DStep& ds) {
     if (!ext_cols_) return Resident();
     Timed tl = TimerStart();

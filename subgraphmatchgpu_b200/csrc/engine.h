@@ -23,6 +23,9 @@ struct DeviceGraph {
   // a neighbour); nhubs x cwords, null when not built
   uint32_t* coarse = nullptr;
   uint32_t cwords = 0;
+  // what k_check_simple found (kNotSimple | kNotSymmetric), -1 not checked;
+  // set at upload for a resident graph
+  int defects = -1;
 };
 
 // Stack allocator over one device allocation.  Levels are processed depth

@@ -237,7 +237,15 @@ struct Step {
   std::vector<uint8_t> sets_after;  // vertices with live candidate sets
   std::string label;
 };
+// A count that a kernel of its own computes per root instead of level by
+// level (the same number; engine.cu decides per run whether the graph and the
+// arena allow it, and runs the steps otherwise).
+enum CountForm : uint8_t {
+  C_STEPS = 0,   // the level program
+  C_CYCLE4 = 1   // Q1: two-path counters (cycle.cuh)
+};
 struct Program {
+  CountForm form = C_STEPS;
   int query_type = 0;
   int n = 0;               // pattern vertices
   int algo = SME_GPU_LIGHT;

@@ -1,0 +1,78 @@
+"""Counts that have kernels of their own (4-cycles by two-path counters)
+against the oracle, closed forms and the level program (an explicit launch
+shape keeps the level program)."""
+import numpy as np
+import pytest
+
+import oracle_py as O
+import subgraphmatchgpu_b200 as sme
+
+pytestmark = pytest.mark.gpu
+ALGOS = [sme.GPU_GPSM, sme.GPU_GPSM_REUSE, sme.GPU_LIGHT]
+
+
+def csr_of(n, edges, both=True):
+    e = np.asarray(edges, dtype=np.int64).reshape(-1, 2)
+    if both:
+        e = np.concatenate([e, e[:, ::-1]])
+    e = np.unique(e, axis=0)
+    rp = np.zeros(n + 1, np.uint64)
+    np.cumsum(np.bincount(e[:, 0], minlength=n), out=rp[1:].view(np.int64))
+    return rp, e[:, 1].astype(np.uint32)
+
+
+def random_edges(n, m, seed):
+    e = np.random.default_rng(seed).integers(0, n, (m, 2))
+    return e[e[:, 0] != e[:, 1]]
+
+
+# the two-path tables: a root of a warp's table (up to 640 two-paths), just
+# above it, the CTA's table, direct counters
+@pytest.mark.parametrize("hubs,leaves", [(2, 300), (2, 639), (2, 641), (3, 400), (8, 700), (5, 6200), (7, 9000)])
+def test_cycles_of_complete_bipartite_graphs(hubs, leaves):
+    edges = [(h, hubs + l) for h in range(hubs) for l in range(leaves)]
+    g = sme.Graph.from_csr(*csr_of(hubs + leaves, edges))
+    want = (hubs * (hubs - 1) // 2) * (leaves * (leaves - 1) // 2)
+    for algo in ALGOS:
+        assert g.count(1, algo) == want
+
+
+@pytest.mark.parametrize("leaves", [50000, 65535, 65536, 110000])
+def test_cycles_over_several_counter_ranges(leaves):
+    # three hubs at the low ids of a graph of more vertices than one range of
+    # 16-bit (98 304) or 32-bit counters (49 152, taken from 65 536 candidates)
+    n = max(leaves + 3, 120001)
+    edges = np.concatenate([np.stack([np.full(leaves, h), np.arange(n - leaves, n)], 1) for h in range(3)])
+    g = sme.Graph.from_csr(*csr_of(n, edges))
+    assert g.count(1) == 3 * (leaves * (leaves - 1) // 2)
+
+
+@pytest.mark.parametrize("scale,ef", [(8, 4), (11, 9), (13, 8)])
+def test_cycles_match_oracle_and_level_program(scale, ef):
+    g = sme.Graph.rmat(scale, ef, seed=scale)
+    rp, cl = g.csr()
+    want = O.count(rp, cl, 1)
+    roots = np.concatenate([np.arange(0, g.n, 3), np.arange(5), np.arange(5)])  # some of them twice
+    part = g.count(1, roots=roots, warp_granularity=1)
+    for resident in (False, True):
+        if resident:
+            g.to_device(0)
+        assert g.count(1) == want
+        assert g.count(1, roots=roots) == part
+        assert g.count(1, root_begin=7, root_end=g.n - 3, root_stride=5) == \
+            g.count(1, root_begin=7, root_end=g.n - 3, root_stride=5, warp_granularity=3)
+
+
+@pytest.mark.parametrize("resident", [False, True])
+def test_graphs_outside_the_contract_keep_the_level_program(resident):
+    # one direction only, or a list with its own vertex: counts as before
+    n = 400
+    e = random_edges(n, 6000, 3)
+    one_way = csr_of(n, e, both=False)
+    loops = csr_of(n, np.concatenate([e, [(5, 5), (9, 9)]]))
+    for rp, cl in (one_way, loops):
+        g = sme.Graph.from_csr(rp, cl)
+        if resident:
+            g.to_device(0)
+        for q in (0, 1, 3, 7):
+            assert g.count(q) == g.count(q, warp_granularity=1), q
