@@ -1,0 +1,455 @@
+// k-cliques (k = 4, 5, 6) of a root task on bit matrices (device code).
+//
+// The level programs of Q3, Q7 and Q11 hold every triangle (and, for the
+// larger cliques, every 4- and 5-clique) as a path and intersect lists once
+// per path.  Here a root's candidates R = N(u0) above u0 (d of them) get a
+// d x d bit matrix of the edges among them, built by one intersection per
+// candidate; the (k-1)-cliques of R are then counted on its rows: k - 3 levels
+// of one AND of two rows each and a last one of AND + popcount.  Rows are
+// triangular (bit j of row i only for i < j), so a clique is counted once.
+// Nothing is materialised and nothing leaves the SM but the count.  Whole
+// calls, level program against this: 4-cliques of R-MAT s18 ef16, every root
+// 73.0 -> 4.5 ms; 5-cliques of the oriented R-MAT s17 ef16 187 -> 19 ms;
+// 4-cliques of 16 384 roots of R-MAT s20 ef16 0.91 -> 0.80 ms.
+//
+// A root's cost grows with d, so roots are sorted into classes by d: up to 32
+// a warp and one word per row (k_clique_small); up to 256, 512 and 1024 (896
+// for k = 6) a CTA with the matrix in shared memory; up to 4096 a CTA with
+// the matrix in global scratch.  A large root's rows are cut into parts that
+// different CTAs take, each with a matrix of its own.
+//
+// ORIENT: the task is every root of a symmetric graph, whose count does not
+// depend on the order of the vertices; the lists are then cut to the
+// neighbours of higher (degree, id) first (k_orient_*), which bounds d by the
+// square root of the stored edges (on R-MAT s18 the largest list falls from 15
+// thousand to a few hundred).  The lists stay sorted by id, the matrix by
+// index.
+#pragma once
+
+#include "cycle.cuh"
+#include "kernels.cuh"
+
+namespace sme {
+namespace dev {
+
+struct CView {
+  DGraph G;
+  const uint2* rng;       // ORIENT: list of v is ocols[rng[v].x .. rng[v].y)
+  const uint32_t* ocols;
+};
+
+template <bool ORIENT>
+__device__ __forceinline__ void CList(const CView& V, uint32_t v, const uint32_t*& a, uint32_t& len) {
+  if (ORIENT) {
+    const uint2 r = __ldg(V.rng + v);
+    a = V.ocols + r.x;
+    len = r.y - r.x;
+  } else {
+    AdjList(V.G, v, a, len);
+  }
+}
+
+// ---- orientation by (degree, id) ------------------------------------------------
+constexpr int ORI_THREADS = 256;
+constexpr uint32_t kOriWarp = 512;                               // edges a warp takes
+constexpr uint32_t kOriTile = kOriWarp * (ORI_THREADS / 32);     // edges a CTA takes
+
+__device__ __forceinline__ bool KeepsEdge(const uint64_t* rp, uint32_t u, uint64_t du, uint32_t x) {
+  const uint64_t dx = __ldg(rp + x + 1) - __ldg(rp + x);
+  return dx > du || (dx == du && x > u);
+}
+
+// FILL 0: kept edges per tile into bs; FILL 1: bs holds their exclusive sums,
+// the kept edges are written to ocols and every list's range to rng (cleared
+// by the caller, so an empty list's range is empty).
+template <bool FILL>
+__global__ void __launch_bounds__(ORI_THREADS) k_orient(const uint64_t* __restrict__ rp,
+                                                        const uint32_t* __restrict__ cols, uint32_t n, uint64_t m,
+                                                        uint64_t* bs, uint32_t* ocols, uint2* rng) {
+  __shared__ uint32_t wkept[ORI_THREADS / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint64_t c0 = (uint64_t)blockIdx.x * kOriTile + (uint64_t)wid * kOriWarp;
+  const uint64_t c1 = c0 + kOriWarp < m ? c0 + kOriWarp : m;
+  uint32_t kept = 0, flags = 0, u0 = 0;
+  if (c0 < m) {
+    u0 = WarpOwner(rp, n, c0);
+    uint32_t u = u0;
+    for (uint32_t k = 0; k < kOriWarp / 32; ++k) {
+      const uint64_t e = c0 + k * 32 + lane;
+      bool keep = false;
+      if (e < c1) {
+        while (__ldg(rp + u + 1) <= e) ++u;  // ends: rp[n] = m > e
+        keep = KeepsEdge(rp, u, __ldg(rp + u + 1) - __ldg(rp + u), __ldg(cols + e));
+      }
+      kept += __popc(__ballot_sync(FULL, keep));
+      flags |= (keep ? 1u : 0u) << k;
+    }
+  }
+  if (lane == 0) wkept[wid] = kept;
+  __syncthreads();
+  if (!FILL) {
+    if (threadIdx.x == 0) {
+      uint32_t t = 0;
+      for (int w = 0; w < ORI_THREADS / 32; ++w) t += wkept[w];
+      bs[blockIdx.x] = t;
+    }
+    return;
+  }
+  uint64_t at = bs[blockIdx.x];
+  for (int w = 0; w < wid; ++w) at += wkept[w];
+  if (c0 >= m) return;
+  uint32_t u = u0;
+  for (uint32_t k = 0; k < kOriWarp / 32; ++k) {
+    const uint64_t e = c0 + k * 32 + lane;
+    const bool keep = (flags >> k) & 1;
+    const unsigned mask = __ballot_sync(FULL, keep);
+    const uint32_t pos = (uint32_t)at + __popc(mask & ((1u << lane) - 1));
+    if (e < c1) {
+      while (__ldg(rp + u + 1) <= e) ++u;
+      if (keep) ocols[pos] = __ldg(cols + e);
+      if (e == __ldg(rp + u)) rng[u].x = pos;
+      if (e + 1 == __ldg(rp + u + 1)) rng[u].y = pos + (keep ? 1 : 0);
+    }
+    at += __popc(mask);
+  }
+}
+
+// ---- classes --------------------------------------------------------------------
+constexpr uint32_t kCliqueS = 32, kCliqueM = 256, kCliqueL = 512, kCliqueG = 4096;
+constexpr uint32_t CliqueX(int k) { return k == 6 ? 896 : 1024; }
+constexpr int kCliqueParts = 8;      // most parts of a root
+constexpr uint32_t kPartShift = 29;  // queue entries: root index | part << 29
+
+// Parts a root of d candidates is cut into: its counting work grows faster
+// than the matrix each part builds.
+__device__ __forceinline__ uint32_t CliqueParts(int k, uint32_t d) {
+  if (d <= kCliqueM) return 1;
+  if (k == 4) return d <= 1024 ? 1 : min(8u, (d + 511) / 512);
+  return min((uint32_t)kCliqueParts, (d + 127) / 128);
+}
+
+struct CliqueQueues {
+  uint32_t* q[5];   // S, M, L, X, G
+  uint32_t cap[5];
+  uint32_t* n;      // entries of each, then the taken ones
+  uint32_t* left;   // roots (vertex ids) above every class
+  uint32_t left_cap;
+  uint32_t* nleft;
+  uint32_t top;     // largest d of class G (of class X when there is no room for scratch)
+  uint32_t* err;
+};
+
+// Sorts the roots into the queues, whose capacities hold every possible entry
+// (one that did not fit would raise the error flag).
+template <int K, bool ORIENT>
+__global__ void __launch_bounds__(256) k_clique_classify(CView V, const uint32_t* __restrict__ roots, uint32_t P,
+                                                         CliqueQueues Q) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t w0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;
+  for (uint32_t base = w0; base < P; base += gridDim.x * blockDim.x) {
+    const uint32_t p = base + lane;
+    uint32_t d = 0, u0 = 0;
+    if (p < P) {
+      u0 = __ldg(roots + p);
+      const uint32_t* a;
+      CList<ORIENT>(V, u0, a, d);
+      if (!ORIENT) d -= LowerBound(a, d, u0 + 1);
+    }
+    int cls = -1;
+    if (d >= K - 1)
+      cls = d <= kCliqueS ? 0 : d <= kCliqueM ? 1 : d <= kCliqueL ? 2 : d <= CliqueX(K) ? 3 : d <= Q.top ? 4 : 5;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const unsigned mask = __ballot_sync(FULL, cls == c);
+      if (!mask) continue;
+      uint32_t at = 0;
+      if (lane == 0) at = atomicAdd(Q.n + c, (uint32_t)__popc(mask));
+      at = __shfl_sync(FULL, at, 0) + __popc(mask & ((1u << lane) - 1));
+      if (cls == c) {
+        if (at < Q.cap[c]) Q.q[c][at] = p;
+        else atomicOr(Q.err, ENGINE_ERR_BOUNDS);
+      }
+    }
+    if (cls >= 2 && cls <= 4) {
+      const uint32_t parts = CliqueParts(K, d);
+      const uint32_t at = atomicAdd(Q.n + cls, parts);
+      for (uint32_t k = 0; k < parts; ++k)
+        if (at + k < Q.cap[cls]) Q.q[cls][at + k] = p | (k << kPartShift);
+        else atomicOr(Q.err, ENGINE_ERR_BOUNDS);
+    }
+    if (cls == 5) {
+      const uint32_t at = atomicAdd(Q.nleft, 1u);
+      if (at < Q.left_cap) Q.left[at] = u0;
+      else atomicOr(Q.err, ENGINE_ERR_BOUNDS);
+    }
+  }
+}
+
+// ---- up to 32 candidates: a warp each ----------------------------------------------
+template <int K>
+__device__ __forceinline__ unsigned long long SmallCliques(const uint32_t* rows, uint32_t s) {
+  // (K)-cliques inside the candidate bits s
+  if constexpr (K == 1) {
+    return __popc(s);
+  } else {
+    unsigned long long c = 0;
+    for (uint32_t b = s; b; b &= b - 1) c += SmallCliques<K - 1>(rows, s & rows[__ffs(b) - 1]);
+    return c;
+  }
+}
+
+// The d(d-1)/2 pairs of candidates are spread over the lanes; a lane finds its
+// pair's edge in the list of the lower one (ORIENT: of the one of lower
+// (degree, id), whose list holds it), by a hub bitmap or a search.
+template <int K, bool ORIENT>
+__global__ void __launch_bounds__(WARP_BLOCK, 6) k_clique_small(CView V, const uint32_t* __restrict__ roots,
+                                                                const uint32_t* __restrict__ q,
+                                                                const uint32_t* __restrict__ nq, uint32_t cap,
+                                                                unsigned long long* acc) {
+  __shared__ uint32_t srows[WARP_BLOCK / 32][32];
+  const int lane = threadIdx.x & 31;
+  uint32_t* rows = srows[threadIdx.x >> 5];
+  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t count = min(*nq, cap);
+  unsigned long long local = 0, bytes = 0;
+  for (uint32_t i = gw; i < count; i += nw) {
+    const uint32_t u0 = __ldg(roots + q[i]);
+    const uint32_t* L;
+    uint32_t d;
+    CList<ORIENT>(V, u0, L, d);
+    if (!ORIENT) {
+      const uint32_t r0 = WarpLowerBound(L, d, u0 + 1);
+      L += r0;
+      d -= r0;
+    }
+    uint32_t x = 0, ln = 0, deg = 0;
+    const uint32_t* lp = nullptr;
+    const uint32_t* bm = nullptr;
+    if (lane < d) {
+      x = __ldg(L + lane);
+      CList<ORIENT>(V, x, lp, ln);
+      if (ORIENT) deg = (uint32_t)(__ldg(V.G.rp + x + 1) - __ldg(V.G.rp + x));
+      else bm = HubBitmap(V.G, x);
+    }
+    rows[lane] = 0;
+    __syncwarp();
+    const uint32_t np = d * (d - 1) / 2;
+    for (uint32_t f0 = 0; f0 < np; f0 += 32) {
+      const uint32_t f = f0 + lane;
+      uint32_t b = (uint32_t)((1.0f + sqrtf(1.0f + 8.0f * (float)f)) * 0.5f);
+      while (b * (b - 1) / 2 > f) --b;
+      while ((b + 1) * b / 2 <= f) ++b;
+      const uint32_t a = f - b * (b - 1) / 2;  // pair a < b
+      const uint32_t xa = __shfl_sync(FULL, x, a & 31), xb = __shfl_sync(FULL, x, b & 31);
+      uint32_t src = a & 31, y = xb;
+      if (ORIENT) {
+        const uint32_t da = __shfl_sync(FULL, deg, a & 31), db = __shfl_sync(FULL, deg, b & 31);
+        if (db < da || (db == da && xb < xa)) {
+          src = b & 31;
+          y = xa;
+        }
+      }
+      const uint64_t sp = __shfl_sync(FULL, (unsigned long long)(uintptr_t)lp, src);
+      const uint32_t sn = __shfl_sync(FULL, ln, src);
+      const uint64_t sb = ORIENT ? 0 : __shfl_sync(FULL, (unsigned long long)(uintptr_t)bm, src);
+      if (f < np) {
+        bool in;
+        if (sb) {
+          in = BitTest(reinterpret_cast<const uint32_t*>(sb), y);
+        } else {
+          const uint32_t* s = reinterpret_cast<const uint32_t*>(sp);
+          const uint32_t pos = LowerBound(s, sn, y);
+          in = pos < sn && __ldg(s + pos) == y;
+        }
+        if (in) atomicOr(rows + a, 1u << b);
+      }
+    }
+    __syncwarp();
+    if (lane < d) local += SmallCliques<K - 2>(rows, rows[lane]);
+    __syncwarp();  // the rows are cleared for the next root
+    if (lane == 0) bytes += 12ULL * d + 8ULL * np;
+  }
+  local = WarpSum(local);
+  if (lane == 0 && local) atomicAdd(acc, local);
+  if (lane == 0 && bytes) atomicAdd(acc + 1, bytes);
+}
+
+// ---- a CTA per root (part) ------------------------------------------------------
+__device__ __forceinline__ uint32_t LowerBoundSmem(const uint32_t* a, uint32_t n, uint32_t x) {
+  const uint32_t* base = a;
+  while (n > 1) {
+    const uint32_t half = n >> 1;
+    base = base[half] < x ? base + half : base;
+    n -= half;
+  }
+  return (uint32_t)(base - a) + (base[0] < x ? 1u : 0u);
+}
+
+// S2 = S & row over words [w0, W) into `out` (zero below w0, when out is
+// given) and the indexes of its bits into `list`; the number of them.
+__device__ __forceinline__ uint32_t AndExpand(const uint32_t* S, const uint32_t* row, uint32_t w0, uint32_t W,
+                                              uint32_t* out, uint16_t* list) {
+  const int lane = threadIdx.x & 31;
+  uint32_t total = 0;
+  for (uint32_t wb = w0 & ~31u; wb < W; wb += 32) {
+    const uint32_t w = wb + lane;
+    uint32_t s = w >= w0 && w < W ? (S ? S[w] & row[w] : row[w]) : 0;
+    if (out && w < W) out[w] = s;
+    const uint32_t c = __popc(s);
+    uint32_t incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += y;
+    }
+    uint32_t at = total + incl - c;
+    for (; s; s &= s - 1) list[at++] = (uint16_t)(w * 32 + (__ffs(s) - 1));
+    total += __shfl_sync(FULL, incl, 31);
+  }
+  return total;
+}
+
+// D-cliques inside the set S, whose nl members `list` holds, on the rows of
+// `mat`; lane-local partial counts.
+template <int D>
+__device__ __forceinline__ unsigned long long RowCliques(const uint32_t* S, const uint16_t* list, uint32_t nl,
+                                                         const uint32_t* mat, uint32_t ws, uint32_t W,
+                                                         uint16_t* lists, uint32_t lcap, uint32_t* sets,
+                                                         uint32_t wcap) {
+  const int lane = threadIdx.x & 31;
+  unsigned long long c = 0;
+  if constexpr (D == 2) {
+    for (uint32_t t = lane; t < nl; t += 32) {
+      const uint32_t l = list[t];
+      const uint32_t* row = mat + (size_t)l * ws;
+      uint32_t s = 0;
+      for (uint32_t w = l >> 5; w < W; ++w) s += __popc(S[w] & row[w]);
+      c += s;
+    }
+  } else {
+    for (uint32_t t = 0; t < nl; ++t) {
+      const uint32_t l = list[t];
+      const uint32_t* row = mat + (size_t)l * ws;
+      __syncwarp();  // the previous round's set and list are read out
+      const uint32_t n2 = AndExpand(S, row, l >> 5, W, sets, lists);
+      __syncwarp();
+      if (n2 >= D - 1)
+        c += RowCliques<D - 1>(sets, lists, n2, mat, ws, W, lists + lcap, lcap, sets + wcap, wcap);
+    }
+  }
+  return c;
+}
+
+// Shared memory of a CTA: the matrix (unless it is in global scratch), the
+// candidates, and per warp K - 3 member lists and K - 4 sets.
+constexpr size_t CliqueSmem(int k, uint32_t dmax, int threads, bool global) {
+  const size_t W = (dmax + 31) / 32, ws = W | 1, warps = threads / 32;
+  return (global ? 0 : (size_t)dmax * ws * 4) + (size_t)dmax * 4 + warps * (k - 4) * (W | 31) * 4 + warps * 4 +
+         warps * (k - 3) * (size_t)dmax * 2 + 64;
+}
+constexpr size_t CliqueScratchWords(uint32_t dmax) { return (size_t)dmax * (((dmax + 31) / 32) | 1); }
+
+template <int K, bool ORIENT, int THREADS, bool GLOBAL>
+__global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t* __restrict__ roots,
+                                                        const uint32_t* __restrict__ q,
+                                                        const uint32_t* __restrict__ nq, uint32_t cap,
+                                                        uint32_t* next, uint32_t dmax, uint32_t* scratch,
+                                                        unsigned long long* acc) {
+  extern __shared__ uint32_t cq_sh[];
+  constexpr int WARPS = THREADS / 32;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const uint32_t wcap = (dmax + 31) / 32;
+  uint32_t* mat = GLOBAL ? scratch + (size_t)blockIdx.x * CliqueScratchWords(dmax) : cq_sh;
+  uint32_t* R = GLOBAL ? cq_sh : cq_sh + (size_t)dmax * (wcap | 1);
+  uint32_t* sets = R + dmax + (size_t)wid * (K - 4) * wcap;
+  uint16_t* lists = reinterpret_cast<uint16_t*>(R + dmax + (size_t)WARPS * (K - 4) * wcap) +
+                    (size_t)wid * (K - 3) * dmax;
+  __shared__ uint32_t s_item, s_row;
+  const uint32_t count = min(*nq, cap);
+  unsigned long long local = 0, bytes = 0;
+  while (true) {
+    if (tid == 0) {
+      s_item = atomicAdd(next, 1u);
+      s_row = 0;
+    }
+    __syncthreads();
+    const uint32_t it = s_item;
+    if (it >= count) break;
+    const uint32_t entry = q[it];
+    const uint32_t u0 = __ldg(roots + (entry & ((1u << kPartShift) - 1)));
+    const uint32_t part = entry >> kPartShift;
+    const uint32_t* L;
+    uint32_t d;
+    CList<ORIENT>(V, u0, L, d);
+    if (!ORIENT) {
+      const uint32_t r0 = WarpLowerBound(L, d, u0 + 1);
+      L += r0;
+      d -= r0;
+    }
+    const uint32_t parts = CliqueParts(K, d);
+    const uint32_t W = (d + 31) / 32, ws = W | 1;  // odd stride: rows spread over the banks
+    for (uint32_t i = tid; i < d; i += THREADS) R[i] = __ldg(L + i);
+    for (uint32_t i = tid; i < d * ws; i += THREADS) mat[i] = 0;
+    __syncthreads();
+    for (uint32_t i = wid; i < d; i += WARPS) {
+      const uint32_t v = R[i];
+      const uint32_t* a;
+      uint32_t len;
+      CList<ORIENT>(V, v, a, len);
+      // index order: either test every later candidate in v's list (one
+      // bitmap word each for a hub, a search else) or look every element of
+      // the list up among the candidates, whichever takes fewer steps
+      const uint32_t* bm = ORIENT ? nullptr : HubBitmap(V.G, v);
+      const uint32_t steps = (d - i + 30) / 32, lg = 32 - __clz(len | 1u);
+      if (!ORIENT && (bm || steps * lg * 2 < (len + 31) / 32)) {
+        for (uint32_t jb = (i + 1) & ~31u; jb < d; jb += 32) {
+          const uint32_t j = jb + lane;
+          bool in = j > i && j < d;
+          if (in) {
+            const uint32_t x = R[j];
+            if (bm) {
+              in = BitTest(bm, x);
+            } else {
+              const uint32_t pos = LowerBound(a, len, x);
+              in = pos < len && __ldg(a + pos) == x;
+            }
+          }
+          const unsigned bits = __ballot_sync(FULL, in);
+          if (lane == 0 && bits) mat[(size_t)i * ws + (jb >> 5)] = bits;  // only this warp writes row i here
+        }
+        if (lane == 0) bytes += 12ULL + 8ULL * (d - i);
+      } else {
+        for (uint32_t e = lane; e < len; e += 32) {
+          const uint32_t x = __ldg(a + e);
+          const uint32_t k = LowerBoundSmem(R, d, x);
+          if (k < d && R[k] == x && (ORIENT || k > i)) {
+            const uint32_t r = min(i, k), c = max(i, k);
+            atomicOr(mat + (size_t)r * ws + (c >> 5), 1u << (c & 31));
+          }
+        }
+        if (lane == 0) bytes += 12ULL + 8ULL * len;
+      }
+    }
+    __syncthreads();
+    while (true) {
+      uint32_t i = 0;
+      if (lane == 0) i = atomicAdd(&s_row, 1u);
+      i = __shfl_sync(FULL, i, 0) * parts + part;
+      if (i >= d) break;
+      const uint32_t* row = mat + (size_t)i * ws;
+      __syncwarp();
+      const uint32_t nl = AndExpand(nullptr, row, i >> 5, W, nullptr, lists);
+      __syncwarp();
+      if (nl >= K - 2)
+        local += RowCliques<K - 2>(row, lists, nl, mat, ws, W, lists + dmax, dmax, sets, wcap);
+    }
+    __syncthreads();  // the matrix is rebuilt for the next root
+  }
+  local = WarpSum(local);
+  if (lane == 0 && local) atomicAdd(acc, local);
+  if (lane == 0 && bytes) atomicAdd(acc + 1, bytes);
+}
+
+}  // namespace dev
+}  // namespace sme

@@ -542,6 +542,7 @@ static CountForm FormOf(const sme_opts& o, const Query& q, const Program& p, boo
       p.steps[0].kind != S_INIT || p.out_slot[p.steps[0].u] != 0)
     return C_STEPS;
   if (q.type == 1) return C_CYCLE4;
+  if (q.n >= 4 && IsOrderedClique(q)) return C_CLIQUE;
   return C_STEPS;
 }
 

@@ -18,9 +18,11 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <cmath>
 #include <cstdio>
 #include <string>
 
+#include "clique.cuh"
 #include "cycle.cuh"
 #include "engine.h"
 #include "kernels.cuh"
@@ -2037,7 +2039,7 @@ class Executor {
       F.P = P;
       F.inst[s0.u] = col;
       ++batches_;
-      if (!CountByForm(col, P)) Level(1, F);
+      if (!CountByForm(task, col, P)) Level(1, F);
       A_.Release(m);
     }
     CK(cudaEventRecord(ev1, st_));
@@ -2124,7 +2126,7 @@ class Executor {
   // and the graph and the arena allow it; false: run the steps.  Below
   // kFormArena of free arena the steps' batches stay in charge, whose budget
   // a caller has set.
-  bool CountByForm(const uint32_t* col, uint32_t P) {
+  bool CountByForm(const RootTask& task, const uint32_t* col, uint32_t P) {
     if (prog_.form == C_STEPS || ext_cols_ || g_.n > 0xFFFFFFFEu || A_.Free() < kFormArena + (uint64_t)P * 8)
       return false;
     if (prog_.form == C_CYCLE4) {
@@ -2132,7 +2134,130 @@ class Executor {
       CountCycles(col, P);
       return true;
     }
-    return false;
+    const bool all = !task.list && task.begin == 0 && task.end >= g_.n && task.stride <= 1 && P == g_.n;
+    const uint32_t bad = Defects(all && !oriented_);
+    if (bad & kNotSimple) return false;
+    const bool orient = all && !oriented_ && !(bad & kNotSymmetric) && g_.m / 2 < 0xFFFFFFFFull;
+    switch (prog_.n) {
+      case 4: return orient ? CountCliques<4, true>(task, col, P) : CountCliques<4, false>(task, col, P);
+      case 5: return orient ? CountCliques<5, true>(task, col, P) : CountCliques<5, false>(task, col, P);
+      case 6: return orient ? CountCliques<6, true>(task, col, P) : CountCliques<6, false>(task, col, P);
+      default: return false;
+    }
+  }
+
+  template <int K, bool ORIENT, int THREADS, bool GLOBAL>
+  void LaunchCliqueClass(const CView& V, const uint32_t* col, const CliqueQueues& Q, int cls, uint32_t dmax,
+                         uint32_t* scratch) {
+    const size_t smem = CliqueSmem(K, dmax, THREADS, GLOBAL);
+    auto kernel = k_clique_cta<K, ORIENT, THREADS, GLOBAL>;
+    // one attribute per instantiation and device (the largest class of it;
+    // setting it twice from two threads is harmless)
+    constexpr size_t kMost = GLOBAL       ? CliqueSmem(K, kCliqueG, THREADS, true)
+                             : THREADS == 128 ? CliqueSmem(K, kCliqueM, THREADS, false)
+                                              : CliqueSmem(K, CliqueX(K), THREADS, false);
+    static std::atomic<int> per_sm_of[64][2];  // resident CTAs: class L or the only one, class X
+    const int dv = ctx_.device, slot = cls == 3 ? 1 : 0;
+    int per_sm = dv >= 0 && dv < 64 ? per_sm_of[dv][slot].load(std::memory_order_acquire) : 0;
+    if (!per_sm) {
+      CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
+      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, THREADS, smem));
+      per_sm = std::max(per_sm, 1);
+      if (dv >= 0 && dv < 64) per_sm_of[dv][slot].store(per_sm, std::memory_order_release);
+    }
+    const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sms_ * (GLOBAL ? 1 : per_sm), Q.cap[cls]);
+    kernel<<<grid, THREADS, smem, st_>>>(V, col, Q.q[cls], Q.n + cls, Q.cap[cls], Q.n + 8 + cls, dmax, scratch,
+                                         ctrl_);
+    Launched();
+  }
+
+  // k-cliques over the roots col[0..P) by bit matrices (clique.cuh).  Roots
+  // above every class run the level program; ORIENT has none to hand back,
+  // so there one such root sends the whole task to it (false).
+  template <int K, bool ORIENT>
+  bool CountCliques(const RootTask& task, const uint32_t* col, uint32_t P) {
+    if (P >= (1u << kPartShift)) return false;
+    // entries a class can hold: distinct roots of more than c candidates are
+    // at most m / c
+    auto most = [&](uint32_t above, uint32_t parts) {
+      const uint64_t roots = task.list ? P : std::min<uint64_t>(P, g_.m / (above + 1) + 1);
+      return (uint32_t)std::min<uint64_t>(roots * parts, 0xFFFFFFFFull);
+    };
+    // largest possible list: ORIENT keeps neighbours of at least the same
+    // degree, so d of them hold d * d of the m stored edges
+    const uint64_t bound = ORIENT ? (uint64_t)std::sqrt((double)g_.m) + 1 : g_.n;
+    CliqueQueues Q{};
+    Q.cap[0] = Q.cap[1] = P;
+    Q.cap[2] = most(kCliqueM, K == 4 ? 1 : 4);
+    Q.cap[3] = most(kCliqueL, K == 4 ? 1 : kCliqueParts);
+    Q.cap[4] = most(CliqueX(K), kCliqueParts);
+    Q.left_cap = most(CliqueX(K), 1);
+    const uint64_t tiles = (g_.m + kOriTile - 1) / kOriTile;
+    uint64_t need = 4096 + Q.left_cap * 4ull;
+    for (int c = 0; c < 5; ++c) need += Q.cap[c] * 4ull + 256;
+    if (ORIENT) need += g_.n * sizeof(uint2) + (g_.m / 2 + 1) * 4 + tiles * 8 + 1024;
+    if (need > A_.Free() / 2) return false;
+    const size_t mark = A_.Mark();
+    uint32_t* ctl = (uint32_t*)A_.Alloc(16 * sizeof(uint32_t));
+    for (int c = 0; c < 5; ++c) Q.q[c] = (uint32_t*)A_.Alloc(std::max<size_t>(Q.cap[c], 1) * 4);
+    Q.left = (uint32_t*)A_.Alloc(std::max<size_t>(Q.left_cap, 1) * 4);
+    Q.n = ctl;
+    Q.nleft = ctl + 5;
+    Q.err = (uint32_t*)(ctrl_ + 3);
+    Q.top = CliqueX(K);
+    uint32_t* scratch = nullptr;
+    const size_t scratch_bytes = (size_t)sms_ * CliqueScratchWords(kCliqueG) * 4;
+    if (bound > Q.top && A_.Free() / 2 > scratch_bytes) Q.top = kCliqueG;
+    CView V{oriented_ ? ViewOf(g_) : Resident(), nullptr, nullptr};
+    CK(cudaMemsetAsync(ctl, 0, 16 * sizeof(uint32_t), st_));
+    paths_ += P;
+    Timed to = TimerStart();
+    if (ORIENT) {
+      uint2* rng = (uint2*)A_.Alloc((size_t)g_.n * sizeof(uint2));
+      uint32_t* ocols = (uint32_t*)A_.Alloc((g_.m / 2 + 1) * 4);
+      uint64_t* bs = (uint64_t*)A_.Alloc(std::max<size_t>(tiles, 1) * 8);
+      CK(cudaMemsetAsync(rng, 0, (size_t)g_.n * sizeof(uint2), st_));
+      if (tiles) {
+        k_orient<false><<<(unsigned)tiles, ORI_THREADS, 0, st_>>>(g_.row_ptrs, g_.cols, (uint32_t)g_.n, g_.m, bs,
+                                                                  ocols, rng);
+        k_scan_partials<<<1, 1024, 0, st_>>>(bs, (uint32_t)tiles);
+        k_orient<true><<<(unsigned)tiles, ORI_THREADS, 0, st_>>>(g_.row_ptrs, g_.cols, (uint32_t)g_.n, g_.m, bs,
+                                                                 ocols, rng);
+        launches_ += 3;
+      }
+      V.rng = rng;
+      V.ocols = ocols;
+    }
+    if (Q.top == kCliqueG) scratch = (uint32_t*)A_.Alloc(scratch_bytes);
+    k_clique_classify<K, ORIENT><<<Grid(P, 256), 256, 0, st_>>>(V, col, P, Q);
+    Launched();
+    TimerStop(to, kPhaseOrganize);
+    uint32_t left = 0;
+    if (bound > Q.top) {  // only then can a root be left
+      left = (uint32_t)ReadU32(Q.nleft);
+      if (left && ORIENT) {
+        A_.Release(mark);
+        paths_ -= P;
+        return false;
+      }
+    }
+    Timed t = TimerStart();
+    // heaviest classes first; a class no list can reach is not launched
+    if (Q.top == kCliqueG) LaunchCliqueClass<K, ORIENT, 256, true>(V, col, Q, 4, kCliqueG, scratch);
+    if (bound > kCliqueL) LaunchCliqueClass<K, ORIENT, 512, false>(V, col, Q, 3, CliqueX(K), nullptr);
+    if (bound > kCliqueM) LaunchCliqueClass<K, ORIENT, 512, false>(V, col, Q, 2, kCliqueL, nullptr);
+    if (bound > kCliqueS) LaunchCliqueClass<K, ORIENT, 128, false>(V, col, Q, 1, kCliqueM, nullptr);
+    k_clique_small<K, ORIENT><<<WarpGrid(P), WARP_BLOCK, 0, st_>>>(V, col, Q.q[0], Q.n, Q.cap[0], ctrl_);
+    Launched();
+    TimerStop(t, kPhaseComputeCount);
+    if (left) {
+      DFront F{};
+      F.P = left;
+      F.inst[prog_.steps[0].u] = Q.left;
+      Level(1, F);
+    }
+    A_.Release(mark);
+    return true;
   }
 
   void CountCycles(const uint32_t* col, uint32_t P) {
@@ -2448,6 +2573,7 @@ class Executor {
   uint32_t heavy_min_ = 2048;  // granularity 4: shortest pivot that gets a CTA
   bool group_by_hub_ = false;  // count steps take their paths hub by hub
   bool use_bitmaps_ = true;
+  bool oriented_ = false;  // each edge once, towards the higher id
   bool root_map_ = true;  // two-list steps on the root's list: k_compute_rootmap
 
  private:
@@ -2748,6 +2874,7 @@ RunResult RunProgram(const Program& prog, const DeviceGraph& g, DeviceContext& c
   Executor ex(prog, g, ctx, d_out, cap);
   ex.gran_ = tuning & 0xff;
   ex.use_bitmaps_ = !(tuning & 0x100);
+  ex.oriented_ = (tuning & 0x200) != 0;
   if (const char* e = std::getenv("SME_HEAVY_PIVOT")) ex.heavy_min_ = (uint32_t)std::max(32L, std::atol(e));
   if (const char* e = std::getenv("SME_GROUP_BY_HUB")) ex.group_by_hub_ = std::atoi(e) != 0;
   if (const char* e = std::getenv("SME_ROOT_MAP")) ex.root_map_ = std::atoi(e) != 0;

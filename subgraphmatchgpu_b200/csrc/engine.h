@@ -95,7 +95,7 @@ RunResult RunProgram(const Program& prog, const DeviceGraph& g, DeviceContext& c
                      uint32_t* d_out, uint64_t cap, int tuning);
 // `tuning`: low byte = intersection launch (0 auto: warp per path,
 // specialised; 1 warp per path generic; 2 flattened, specialised; 3 as 0 at
-// six blocks per SM); bit 8 set = no hub bitmaps.
+// six blocks per SM); bit 8 set = no hub bitmaps, bit 9 = an oriented graph.
 inline int Tuning(const sme_opts& o) { return (o.warp_granularity & 0xff) | (o.list_only ? 0x100 : 0); }
 // The launch for a graph: the auto choice (granularity 0) takes the
 // flattened kernel on an oriented graph, whose lists are short (the
@@ -106,6 +106,7 @@ inline int Tuning(const sme_opts& o) { return (o.warp_granularity & 0xff) | (o.l
 inline int TuningFor(const sme_opts& o, const HostGraph& g) {
   int t = Tuning(o);
   if ((t & 0xff) == 0 && g.oriented) t |= 2;
+  if (g.oriented) t |= 0x200;
   return t;
 }
 

@@ -242,7 +242,8 @@ struct Step {
 // arena allow it, and runs the steps otherwise).
 enum CountForm : uint8_t {
   C_STEPS = 0,   // the level program
-  C_CYCLE4 = 1   // Q1: two-path counters (cycle.cuh)
+  C_CYCLE4 = 1,  // Q1: two-path counters (cycle.cuh)
+  C_CLIQUE = 2   // Q3, Q7, Q11: bit matrices per root (clique.cuh)
 };
 struct Program {
   CountForm form = C_STEPS;

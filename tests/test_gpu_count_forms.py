@@ -1,6 +1,9 @@
-"""Counts that have kernels of their own (4-cycles by two-path counters)
+"""Counts that have kernels of their own (4-cycles by two-path counters,
+cliques on bit matrices)
 against the oracle, closed forms and the level program (an explicit launch
 shape keeps the level program)."""
+from math import comb
+
 import numpy as np
 import pytest
 
@@ -76,3 +79,55 @@ def test_graphs_outside_the_contract_keep_the_level_program(resident):
             g.to_device(0)
         for q in (0, 1, 3, 7):
             assert g.count(q) == g.count(q, warp_granularity=1), q
+
+
+# class edges of the bit matrices: a root of a complete graph of n vertices
+# has n - 1 candidates
+@pytest.mark.parametrize("n,ks", [(4, (4, 5)), (5, (4, 5, 6)), (33, (4, 5, 6)), (34, (4, 5, 6)), (65, (4, 5, 6)),
+                                  (130, (4, 5, 6)), (257, (4, 5)), (258, (4, 5)), (513, (4, 5)), (514, (4,)),
+                                  (1025, (4,)), (1026, (4,))])
+def test_cliques_of_complete_graphs(n, ks):
+    g = sme.Graph.clique(n)
+    g.to_device(0)
+    o, _ = g.degree_order(orient=True)
+    for k in ks:
+        q = {4: 3, 5: 7, 6: 11}[k]
+        assert g.count(q) == comb(n, k)
+        assert o.count(q) == comb(n, k)
+        # root 0 has n - 1 candidates, root 1 one fewer
+        assert g.count(q, roots=[1, 0, 1]) == comb(n - 1, k - 1) + 2 * comb(n - 2, k - 1)
+
+
+# vertex 0 sees every other vertex: a root of d candidates in every class, and
+# above the last one, which keeps the level program
+@pytest.mark.parametrize("d", [31, 256, 257, 700, 896, 897, 1024, 1025, 4096, 4097, 5000])
+@pytest.mark.parametrize("q", [3, 7, 11])
+def test_cliques_of_a_hub_root(d, q):
+    e = np.concatenate([np.stack([np.zeros(d, np.int64), np.arange(1, d + 1)], 1), 1 + random_edges(d, 14 * d, d)])
+    rng = np.random.default_rng(d)
+    core = rng.choice(np.arange(1, d + 1), min(d, 40), replace=False)
+    a, b = np.triu_indices(len(core), 1)
+    e = np.concatenate([e, np.stack([core[a], core[b]], 1)])
+    rp, cl = csr_of(d + 1, e)
+    g = sme.Graph.from_csr(rp, cl)
+    g.to_device(0)
+    want = g.count(q, warp_granularity=1)
+    assert want > 0
+    assert g.count(q) == want
+    roots = [0, 3, 0, d]
+    assert g.count(q, roots=roots) == g.count(q, roots=roots, warp_granularity=1)
+
+
+@pytest.mark.parametrize("resident", [False, True])
+def test_cliques_of_skewed_graphs(resident):
+    g = sme.Graph.rmat(14, 12, seed=2)
+    o, _ = g.degree_order(orient=True)
+    renumbered, _ = g.degree_order(orient=False)
+    for x in (g, o, renumbered) if resident else ():
+        x.to_device(0)
+    for q in (3, 7):
+        want = g.count(q, warp_granularity=3)
+        assert [x.count(q, a) for x in (g, o, renumbered) for a in ALGOS] == [want] * 9
+        part = dict(root_begin=5, root_end=g.n - 9, root_stride=3)
+        assert g.count(q, **part) == g.count(q, warp_granularity=3, **part)
+        assert o.count(q, **part) == o.count(q, warp_granularity=2, **part)
