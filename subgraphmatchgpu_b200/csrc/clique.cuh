@@ -9,8 +9,16 @@
 // triangular (bit j of row i only for i < j), so a clique is counted once.
 // Nothing is materialised and nothing leaves the SM but the count.  Whole
 // calls, level program against this: 4-cliques of R-MAT s18 ef16, every root
-// 73.0 -> 4.5 ms; 5-cliques of the oriented R-MAT s17 ef16 187 -> 19 ms;
-// 4-cliques of 16 384 roots of R-MAT s20 ef16 0.91 -> 0.80 ms.
+// 73.0 -> 2.2 ms; 5-cliques of the oriented R-MAT s17 ef16 187 -> 8.5 ms;
+// 4-cliques of 16 384 roots of R-MAT s20 ef16 0.91 -> 0.40 ms.
+//
+// Few roots are bound by the latency of the build's loads (hub bitmap words
+// from HBM): hence four of them in flight per lane, 32 lists fetched at once
+// and many warps per root (4-cliques, s20 roots: 0.80 -> 0.40 ms).  Many roots
+// are bound by instruction issue: hence the candidates' hash table (1-2
+// shared-memory reads per looked-up element, a binary search takes 8) and the
+// member lists compacted from their parent's by ballot (5-cliques, s17: 18 ->
+// 8.5 ms together; expanding the bits of every AND took the other half).
 //
 // A root's cost grows with d, so roots are sorted into classes by d: up to 32
 // a warp and one word per row (k_clique_small); up to 256, 512 and 1024 (896
@@ -116,6 +124,7 @@ __global__ void __launch_bounds__(ORI_THREADS) k_orient(const uint64_t* __restri
 
 // ---- classes --------------------------------------------------------------------
 constexpr uint32_t kCliqueS = 32, kCliqueM = 256, kCliqueL = 512, kCliqueG = 4096;
+constexpr int kCliqueMThreads = 256;
 constexpr uint32_t CliqueX(int k) { return k == 6 ? 896 : 1024; }
 constexpr int kCliqueParts = 8;      // most parts of a root
 constexpr uint32_t kPartShift = 29;  // queue entries: root index | part << 29
@@ -286,16 +295,35 @@ __device__ __forceinline__ uint32_t LowerBoundSmem(const uint32_t* a, uint32_t n
   return (uint32_t)(base - a) + (base[0] < x ? 1u : 0u);
 }
 
-// S2 = S & row over words [w0, W) into `out` (zero below w0, when out is
-// given) and the indexes of its bits into `list`; the number of them.
-__device__ __forceinline__ uint32_t AndExpand(const uint32_t* S, const uint32_t* row, uint32_t w0, uint32_t W,
-                                              uint32_t* out, uint16_t* list) {
+// The candidates' positions by value: an open-addressed table of 2^lg slots,
+// at most half full.  Most looked-up values are no candidate and stop at the
+// first free slot, where a binary search takes log2(d) dependent steps.
+__device__ __forceinline__ uint32_t TableSlot(uint32_t x, uint32_t lg) { return (x * 2654435761u) >> (32 - lg); }
+__device__ __forceinline__ void TablePut(uint32_t* keys, uint16_t* at, uint32_t lg, uint32_t x, uint32_t i) {
+  uint32_t h = TableSlot(x, lg);
+  while (atomicCAS(keys + h, kNoKey, x) != kNoKey) h = (h + 1) & ((1u << lg) - 1);
+  at[h] = (uint16_t)i;
+}
+// Position of x, or kNoKey.
+__device__ __forceinline__ uint32_t TableGet(const uint32_t* keys, const uint16_t* at, uint32_t lg, uint32_t x) {
+  uint32_t h = TableSlot(x, lg);
+  while (true) {
+    const uint32_t k = keys[h];
+    if (k == x) return at[h];
+    if (k == kNoKey) return kNoKey;
+    h = (h + 1) & ((1u << lg) - 1);
+  }
+}
+constexpr uint32_t TableLg(uint32_t dmax) { return dmax <= 256 ? 10 : 11; }
+
+// The indexes of the bits of words [w0, W) of `row` into `list`; the number
+// of them.
+__device__ __forceinline__ uint32_t Expand(const uint32_t* row, uint32_t w0, uint32_t W, uint16_t* list) {
   const int lane = threadIdx.x & 31;
   uint32_t total = 0;
   for (uint32_t wb = w0 & ~31u; wb < W; wb += 32) {
     const uint32_t w = wb + lane;
-    uint32_t s = w >= w0 && w < W ? (S ? S[w] & row[w] : row[w]) : 0;
-    if (out && w < W) out[w] = s;
+    uint32_t s = w >= w0 && w < W ? row[w] : 0;
     const uint32_t c = __popc(s);
     uint32_t incl = c;
 #pragma unroll
@@ -324,15 +352,26 @@ __device__ __forceinline__ unsigned long long RowCliques(const uint32_t* S, cons
       const uint32_t l = list[t];
       const uint32_t* row = mat + (size_t)l * ws;
       uint32_t s = 0;
+#pragma unroll 4
       for (uint32_t w = l >> 5; w < W; ++w) s += __popc(S[w] & row[w]);
       c += s;
     }
   } else {
-    for (uint32_t t = 0; t < nl; ++t) {
+    for (uint32_t t = 0; t + D - 1 < nl; ++t) {
       const uint32_t l = list[t];
       const uint32_t* row = mat + (size_t)l * ws;
       __syncwarp();  // the previous round's set and list are read out
-      const uint32_t n2 = AndExpand(S, row, l >> 5, W, sets, lists);
+      for (uint32_t w = (l >> 5) + lane; w < W; w += 32) sets[w] = S[w] & row[w];
+      // the members after l that l is joined to
+      uint32_t n2 = 0;
+      for (uint32_t k0 = t + 1; k0 < nl; k0 += 32) {
+        const uint32_t k = k0 + lane;
+        const uint32_t x = k < nl ? list[k] : 0;
+        const bool in = k < nl && ((row[x >> 5] >> (x & 31)) & 1u);
+        const unsigned mask = __ballot_sync(FULL, in);
+        if (in) lists[n2 + __popc(mask & ((1u << lane) - 1))] = (uint16_t)x;
+        n2 += __popc(mask);
+      }
       __syncwarp();
       if (n2 >= D - 1)
         c += RowCliques<D - 1>(sets, lists, n2, mat, ws, W, lists + lcap, lcap, sets + wcap, wcap);
@@ -342,10 +381,11 @@ __device__ __forceinline__ unsigned long long RowCliques(const uint32_t* S, cons
 }
 
 // Shared memory of a CTA: the matrix (unless it is in global scratch), the
-// candidates, and per warp K - 3 member lists and K - 4 sets.
+// candidates and their table (not with the matrix in scratch), and per warp
+// K - 3 member lists and K - 4 sets.
 constexpr size_t CliqueSmem(int k, uint32_t dmax, int threads, bool global) {
   const size_t W = (dmax + 31) / 32, ws = W | 1, warps = threads / 32;
-  return (global ? 0 : (size_t)dmax * ws * 4) + (size_t)dmax * 4 + warps * (k - 4) * (W | 31) * 4 + warps * 4 +
+  return (global ? 0 : (size_t)dmax * ws * 4) + (size_t)dmax * 4 + warps * (k - 4) * W * 4 + (global ? 0 : (size_t)6 << TableLg(dmax)) +
          warps * (k - 3) * (size_t)dmax * 2 + 64;
 }
 constexpr size_t CliqueScratchWords(uint32_t dmax) { return (size_t)dmax * (((dmax + 31) / 32) | 1); }
@@ -362,8 +402,12 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
   const uint32_t wcap = (dmax + 31) / 32;
   uint32_t* mat = GLOBAL ? scratch + (size_t)blockIdx.x * CliqueScratchWords(dmax) : cq_sh;
   uint32_t* R = GLOBAL ? cq_sh : cq_sh + (size_t)dmax * (wcap | 1);
-  uint32_t* sets = R + dmax + (size_t)wid * (K - 4) * wcap;
-  uint16_t* lists = reinterpret_cast<uint16_t*>(R + dmax + (size_t)WARPS * (K - 4) * wcap) +
+  const uint32_t tlg = TableLg(dmax);
+  uint32_t* keys = R + dmax;
+  uint16_t* at = reinterpret_cast<uint16_t*>(keys + (1u << tlg));
+  uint32_t* sets0 = GLOBAL ? R + dmax : keys + (3u << (tlg - 1));
+  uint32_t* sets = sets0 + (size_t)wid * (K - 4) * wcap;
+  uint16_t* lists = reinterpret_cast<uint16_t*>(sets0 + (size_t)WARPS * (K - 4) * wcap) +
                     (size_t)wid * (K - 3) * dmax;
   __shared__ uint32_t s_item, s_row;
   const uint32_t count = min(*nq, cap);
@@ -391,44 +435,87 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
     const uint32_t W = (d + 31) / 32, ws = W | 1;  // odd stride: rows spread over the banks
     for (uint32_t i = tid; i < d; i += THREADS) R[i] = __ldg(L + i);
     for (uint32_t i = tid; i < d * ws; i += THREADS) mat[i] = 0;
+    if (!GLOBAL) {
+      for (uint32_t i = tid; i < (1u << tlg); i += THREADS) keys[i] = kNoKey;
+      __syncthreads();
+      for (uint32_t i = tid; i < d; i += THREADS) TablePut(keys, at, tlg, R[i], i);
+    }
     __syncthreads();
-    for (uint32_t i = wid; i < d; i += WARPS) {
-      const uint32_t v = R[i];
-      const uint32_t* a;
-      uint32_t len;
-      CList<ORIENT>(V, v, a, len);
-      // index order: either test every later candidate in v's list (one
-      // bitmap word each for a hub, a search else) or look every element of
-      // the list up among the candidates, whichever takes fewer steps
-      const uint32_t* bm = ORIENT ? nullptr : HubBitmap(V.G, v);
-      const uint32_t steps = (d - i + 30) / 32, lg = 32 - __clz(len | 1u);
-      if (!ORIENT && (bm || steps * lg * 2 < (len + 31) / 32)) {
-        for (uint32_t jb = (i + 1) & ~31u; jb < d; jb += 32) {
-          const uint32_t j = jb + lane;
-          bool in = j > i && j < d;
-          if (in) {
-            const uint32_t x = R[j];
-            if (bm) {
-              in = BitTest(bm, x);
-            } else {
-              const uint32_t pos = LowerBound(a, len, x);
-              in = pos < len && __ldg(a + pos) == x;
+    // rows wid, wid + WARPS, ...: the lanes fetch the lists of 32 rows at a
+    // time, then the warp builds them one by one, four loads in flight per
+    // lane (the loads are what a row waits for)
+    for (uint32_t i0 = wid; i0 < d; i0 += WARPS * 32) {
+      const uint32_t mine = i0 + lane * WARPS;
+      const uint32_t* ma = nullptr;
+      const uint32_t* mb = nullptr;
+      uint32_t mlen = 0;
+      if (mine < d) {
+        CList<ORIENT>(V, R[mine], ma, mlen);
+        if (!ORIENT) mb = HubBitmap(V.G, R[mine]);
+      }
+      const uint32_t rows = min(32u, (d - i0 + WARPS - 1) / WARPS);
+      for (uint32_t k = 0; k < rows; ++k) {
+        const uint32_t i = i0 + k * WARPS;
+        const uint32_t* a = reinterpret_cast<const uint32_t*>(__shfl_sync(FULL, (unsigned long long)(uintptr_t)ma, k));
+        const uint32_t len = __shfl_sync(FULL, mlen, k);
+        const uint32_t* bm =
+            ORIENT ? nullptr
+                   : reinterpret_cast<const uint32_t*>(__shfl_sync(FULL, (unsigned long long)(uintptr_t)mb, k));
+        // index order: either test every later candidate in v's list (one
+        // bitmap word each for a hub, a search else) or look every element of
+        // the list up among the candidates, whichever takes fewer steps
+        const uint32_t steps = (d - i + 30) / 32, lg = 32 - __clz(len | 1u);
+        if (!ORIENT && bm) {
+          for (uint32_t jb = (i + 1) & ~31u; jb < d; jb += 128) {
+            uint32_t x[4], word[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+              const uint32_t j = jb + t * 32 + lane;
+              x[t] = j < d ? R[j] : 0;
+              word[t] = j > i && j < d ? __ldg(bm + (x[t] >> 5)) : 0;
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+              const unsigned bits = __ballot_sync(FULL, (word[t] >> (x[t] & 31)) & 1u);
+              if (lane == 0 && bits) mat[(size_t)i * ws + (jb >> 5) + t] = bits;  // only this warp writes row i here
             }
           }
-          const unsigned bits = __ballot_sync(FULL, in);
-          if (lane == 0 && bits) mat[(size_t)i * ws + (jb >> 5)] = bits;  // only this warp writes row i here
-        }
-        if (lane == 0) bytes += 12ULL + 8ULL * (d - i);
-      } else {
-        for (uint32_t e = lane; e < len; e += 32) {
-          const uint32_t x = __ldg(a + e);
-          const uint32_t k = LowerBoundSmem(R, d, x);
-          if (k < d && R[k] == x && (ORIENT || k > i)) {
-            const uint32_t r = min(i, k), c = max(i, k);
-            atomicOr(mat + (size_t)r * ws + (c >> 5), 1u << (c & 31));
+          if (lane == 0) bytes += 12ULL + 8ULL * (d - i);
+        } else if (!ORIENT && steps * lg * 2 < (len + 31) / 32) {
+          for (uint32_t jb = (i + 1) & ~31u; jb < d; jb += 32) {
+            const uint32_t j = jb + lane;
+            bool in = j > i && j < d;
+            if (in) {
+              const uint32_t x = R[j], pos = LowerBound(a, len, x);
+              in = pos < len && __ldg(a + pos) == x;
+            }
+            const unsigned bits = __ballot_sync(FULL, in);
+            if (lane == 0 && bits) mat[(size_t)i * ws + (jb >> 5)] = bits;
           }
+          if (lane == 0) bytes += 12ULL + 8ULL * (d - i);
+        } else {
+          for (uint32_t e0 = lane; e0 < len; e0 += 128) {
+            uint32_t x[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) x[t] = e0 + t * 32 < len ? __ldg(a + e0 + t * 32) : 0xFFFFFFFFu;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+              if (e0 + t * 32 >= len) break;
+              uint32_t c;
+              if (GLOBAL) {
+                c = LowerBoundSmem(R, d, x[t]);
+                if (c < d && R[c] != x[t]) c = d;
+              } else {
+                c = TableGet(keys, at, tlg, x[t]);
+              }
+              if (c < d && (ORIENT || c > i)) {
+                const uint32_t lo = min(i, c), hi = max(i, c);
+                atomicOr(mat + (size_t)lo * ws + (hi >> 5), 1u << (hi & 31));
+              }
+            }
+          }
+          if (lane == 0) bytes += 12ULL + 8ULL * len;
         }
-        if (lane == 0) bytes += 12ULL + 8ULL * len;
       }
     }
     __syncthreads();
@@ -439,7 +526,7 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
       if (i >= d) break;
       const uint32_t* row = mat + (size_t)i * ws;
       __syncwarp();
-      const uint32_t nl = AndExpand(nullptr, row, i >> 5, W, nullptr, lists);
+      const uint32_t nl = Expand(row, i >> 5, W, lists);
       __syncwarp();
       if (nl >= K - 2)
         local += RowCliques<K - 2>(row, lists, nl, mat, ws, W, lists + dmax, dmax, sets, wcap);

@@ -13,7 +13,8 @@
 // What bounds it: one list element read (L2) and one shared-memory atomic per
 // two-path, against a search or a walk of dozens of elements per two-path in
 // the level program.  Whole calls, level program against this: R-MAT s20
-// ef16, 512 roots of degree <= 1024 (9 300 two-paths a root) 3.79 -> 0.47 ms;
+// ef16, 512 roots of degree <= 1024 (9 300 two-paths a root) 3.79 -> 0.27 ms
+// (0.47 with a root's counter ranges one after another in one CTA);
 // a Barabasi-Albert graph of 30 011 vertices and 9 edges a vertex, every root
 // (113 two-paths a root) 3.83 -> 0.23 ms.
 #pragma once
@@ -111,6 +112,7 @@ constexpr int CYW_THREADS = 512;
 constexpr int CYW_WARPS = CYW_THREADS / 32;
 constexpr uint32_t kCycleWarpLg = 10;
 constexpr uint32_t kCycleWarpMax = 640;
+constexpr uint32_t kCycleWarpCand = 64;  // a warp searches 32 lists at a time, a CTA 1024
 constexpr size_t kCycleWarpSmem = (size_t)CYW_WARPS * ((4u << kCycleWarpLg) + (2u << kCycleWarpLg));
 
 // The part of u1's list above u0 (u1 = the i-th candidate), per lane.
@@ -143,7 +145,7 @@ __global__ void __launch_bounds__(CYW_THREADS, 2) k_cycle4_warp(DGraph G, const 
     L += r0;
     d -= r0;
     const uint32_t* a = nullptr;
-    uint32_t len = 0, total = 0;
+    uint32_t len = 0, total = d > kCycleWarpCand ? kCycleWarpMax + 1 : 0;
     for (uint32_t i0 = 0; i0 < d && total <= kCycleWarpMax; i0 += 32) {
       len = 0;
       if (i0 + lane < d) TwoPathRange(G, __ldg(L + i0 + lane), u0, a, len);
@@ -199,12 +201,14 @@ __global__ void __launch_bounds__(CYW_THREADS, 2) k_cycle4_warp(DGraph G, const 
   if (lane == 0 && bytes) atomicAdd(acc + 1, bytes);
 }
 
-// Roots with more two-paths: one CTA each.  Up to kCycleHashMax two-paths go
-// through one table in shared memory; more of them are counted in direct
-// 16-bit counters (32-bit ones when the root has 65536 or more candidates),
-// one range of w at a time.  Neighbours are taken 1024 at a time, one per
-// thread; their clipped lists are concatenated and cut into segments of
-// kCycleSeg elements, a warp finding a segment's first list by one search.
+// Roots with more two-paths.  Up to kCycleHashMax of them go through one
+// table in a CTA's shared memory (TILED 0).  More are counted in direct 16-bit
+// counters (32-bit ones when the root has 65536 or more candidates), one
+// range of w at a time; the ranges are independent, so they are queued and
+// different CTAs take them (TILED 1).  Neighbours are taken 1024 at a time,
+// one per thread; their clipped lists are concatenated and cut into segments
+// of kCycleSeg elements, a warp finding a segment's first list by one search
+// and keeping four loads in flight per lane.
 constexpr int CYC_THREADS = 1024;
 constexpr uint32_t kCycleHashLg = 15;
 constexpr uint32_t kCycleHashMax = 24576;  // 3/4 of the slots
@@ -235,102 +239,118 @@ __device__ __forceinline__ uint64_t CtaInclusive(uint64_t v, uint64_t* wtot) {
   return v + (wid ? wtot[wid - 1] : 0);
 }
 
+// Entries of `tiles`: queued root index << 32 | range.
+template <bool TILED>
 __global__ void __launch_bounds__(CYC_THREADS, 1) k_cycle4_cta(DGraph G, uint32_t n,
                                                                const uint32_t* __restrict__ roots,
                                                                const uint32_t* __restrict__ queue,
                                                                const uint32_t* __restrict__ nqueue, uint32_t* next,
-                                                               unsigned long long* acc) {
+                                                               uint64_t* tiles, uint32_t* ntiles, uint32_t tiles_cap,
+                                                               uint32_t* err, unsigned long long* acc) {
   extern __shared__ uint64_t cyc_sh[];
-  uint64_t* off = cyc_sh;                        // exclusive offsets of the chunk's lists, then their sum
-  uint64_t* ptr = off + CYC_THREADS + 2;         // first element of each (16-byte aligned, as is the table)
+  uint64_t* off = cyc_sh;                 // exclusive offsets of the chunk's lists, then their sum
+  uint64_t* ptr = off + CYC_THREADS + 2;  // first element of each (16-byte aligned, as is the table)
   uint32_t* table = reinterpret_cast<uint32_t*>(ptr + CYC_THREADS);
   __shared__ uint64_t wtot[32];
   __shared__ uint32_t s_item;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const uint32_t nq = *nqueue;
+  const uint32_t nq = TILED ? min(*ntiles, tiles_cap) : *nqueue;
   unsigned long long local = 0, bytes = 0;
   while (true) {
     if (tid == 0) s_item = atomicAdd(next, 1u);
     __syncthreads();
     const uint32_t it = s_item;
     if (it >= nq) break;
-    const uint32_t u0 = __ldg(roots + queue[it]);
+    const uint32_t slot = TILED ? (uint32_t)(tiles[it] >> 32) : it;
+    const uint32_t u0 = __ldg(roots + queue[slot]);
     const uint32_t* L;
     uint32_t d;
     AdjList(G, u0, L, d);
     const uint32_t r0 = WarpLowerBound(L, d, u0 + 1);
     L += r0;
     d -= r0;
-    // two-paths of the root (the last chunk's ranges stay in registers)
+    const bool wide = d > 0xFFFFu;
+    const uint64_t tile = kCycleTable / (wide ? 4 : 2);  // counters per range
     const uint32_t* a = nullptr;
-    uint32_t len = 0;
-    uint64_t mine = 0;
-    for (uint32_t i = tid; i < d; i += CYC_THREADS) {
-      TwoPathRange(G, __ldg(L + i), u0, a, len);
-      mine += len;
-    }
-    CtaInclusive(mine, wtot);
-    const uint64_t total = wtot[31];
-    __syncthreads();  // wtot is rewritten
-    const bool hash = total <= kCycleHashMax;
-    const bool wide = !hash && d > 0xFFFFu;
-    uint32_t lg = 0;
-    uint64_t tile = 0, first = 0, last = 1;  // ranges [first + t tile, ...) of w (hash: one)
-    uint32_t clear = 0;                      // 16-byte quads of the table in use
-    if (hash) {
-      lg = 10;
+    uint32_t len = 0, lg = 10, clear, nkeys = 0;
+    uint64_t t0 = 0, t1 = 0;
+    if (TILED) {
+      t0 = (uint64_t)u0 + 1 + (uint32_t)tiles[it] * tile;
+      t1 = t0 + tile < n ? t0 + tile : n;
+      clear = (uint32_t)(((t1 - t0) * (wide ? 4 : 2) + 15) / 16);
+    } else {
+      // two-paths of the root (ranges of up to 1024 candidates stay in registers)
+      uint64_t mine = 0;
+      for (uint32_t i = tid; i < d; i += CYC_THREADS) {
+        TwoPathRange(G, __ldg(L + i), u0, a, len);
+        mine += len;
+      }
+      CtaInclusive(mine, wtot);
+      const uint64_t total = wtot[31];
+      __syncthreads();  // wtot and s_item are rewritten
+      if (tid == 0) bytes += 12ULL * d + 4ULL * total;
+      if (total > kCycleHashMax) {
+        const uint32_t ranges = (uint32_t)((n - 1 - (uint64_t)u0 + tile - 1) / tile);
+        if (tid == 0) {
+          const uint32_t at = atomicAdd(ntiles, ranges);
+          for (uint32_t k = 0; k < ranges; ++k)
+            if (at + k < tiles_cap) tiles[at + k] = (uint64_t)slot << 32 | k;
+            else atomicOr(err, ENGINE_ERR_BOUNDS);
+        }
+        continue;
+      }
       while ((3u << lg) / 4 < total) ++lg;  // <= kCycleHashLg
       clear = (6u << lg) / 16;
-    } else {
-      tile = kCycleTable / (wide ? 4 : 2);
-      first = (uint64_t)u0 + 1;
-      last = n;
-      const uint64_t span = last - first < tile ? last - first : tile;
-      clear = (uint32_t)((span * (wide ? 4 : 2) + 15) / 16);
+      nkeys = (4u << lg) / 16;
     }
-    uint32_t* cnt = table + (hash ? 1u << lg : 0);
-    if (tid == 0) bytes += 12ULL * d + 4ULL * total;
-    for (uint64_t t0 = first; t0 < last; t0 += hash ? 1 : tile) {
-      const uint64_t t1 = hash || t0 + tile > last ? last : t0 + tile;
-      uint4* q = reinterpret_cast<uint4*>(table);
-      const uint32_t nkeys = hash ? (4u << lg) / 16 : 0;
-      for (uint32_t i = tid; i < clear; i += CYC_THREADS)
-        q[i] = i < nkeys ? make_uint4(kNoKey, kNoKey, kNoKey, kNoKey) : make_uint4(0, 0, 0, 0);
-      for (uint32_t i0 = 0; i0 < d; i0 += CYC_THREADS) {
-        if (!(hash && d <= CYC_THREADS)) {  // else the registers hold the only chunk
-          len = 0;
-          if (i0 + tid < d) {
-            TwoPathRange(G, __ldg(L + i0 + tid), u0, a, len);
-            if (!hash) {
-              const uint32_t s0 = LowerBound(a, len, (uint32_t)t0);
-              const uint32_t s1 = t1 >= n ? len : s0 + LowerBound(a + s0, len - s0, (uint32_t)t1);
-              a += s0;
-              len = s1 - s0;
+    uint32_t* cnt = table + (1u << lg);  // hash: counters after the keys
+    uint4* q = reinterpret_cast<uint4*>(table);
+    for (uint32_t i = tid; i < clear; i += CYC_THREADS)
+      q[i] = i < nkeys ? make_uint4(kNoKey, kNoKey, kNoKey, kNoKey) : make_uint4(0, 0, 0, 0);
+    for (uint32_t i0 = 0; i0 < d; i0 += CYC_THREADS) {
+      if (TILED) {
+        len = 0;
+        if (i0 + tid < d) {
+          AdjList(G, __ldg(L + i0 + tid), a, len);
+          const uint32_t s0 = LowerBound(a, len, (uint32_t)t0);
+          const uint32_t s1 = t1 >= n ? len : LowerBound(a, len, (uint32_t)t1);
+          a += s0;
+          len = s1 - s0;
+        }
+      } else if (d > CYC_THREADS) {
+        len = 0;
+        if (i0 + tid < d) TwoPathRange(G, __ldg(L + i0 + tid), u0, a, len);
+      }
+      const uint64_t incl = CtaInclusive(len, wtot);
+      off[tid] = incl - len;
+      ptr[tid] = (uint64_t)(uintptr_t)a;
+      const uint64_t sum = wtot[31];
+      if (tid == 0) off[CYC_THREADS] = sum;
+      __syncthreads();  // offsets, pointers and the cleared table are visible
+      for (uint64_t f0 = (uint64_t)wid * kCycleSeg; f0 < sum; f0 += (uint64_t)(CYC_THREADS / 32) * kCycleSeg) {
+        // last list whose offset is <= f0 (uniform in the warp)
+        int j = 0;
+#pragma unroll
+        for (int o = CYC_THREADS / 2; o > 0; o >>= 1)
+          if (off[j + o] <= f0) j += o;
+        const uint64_t f1 = f0 + kCycleSeg < sum ? f0 + kCycleSeg : sum;
+        for (uint64_t f = f0 + lane; f < f1; f += 128) {
+          uint32_t w[4];
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const uint64_t g = f + 32 * t;
+            if (g < f1) {
+              while (off[j + 1] <= g) ++j;  // ends: off[CYC_THREADS] = sum > g
+              w[t] = __ldg(reinterpret_cast<const uint32_t*>(ptr[j]) + (g - off[j]));
             }
           }
-        } else if (tid >= d) {
-          len = 0;
-        }
-        const uint64_t incl = CtaInclusive(len, wtot);
-        off[tid] = incl - len;
-        ptr[tid] = (uint64_t)(uintptr_t)a;
-        const uint64_t sum = wtot[31];
-        if (tid == 0) off[CYC_THREADS] = sum;
-        __syncthreads();  // offsets, pointers and the cleared table are visible
-        for (uint64_t f0 = (uint64_t)wid * kCycleSeg; f0 < sum; f0 += (uint64_t)(CYC_THREADS / 32) * kCycleSeg) {
-          // last list whose offset is <= f0 (uniform in the warp)
-          int j = 0;
 #pragma unroll
-          for (int o = CYC_THREADS / 2; o > 0; o >>= 1)
-            if (off[j + o] <= f0) j += o;
-          const uint64_t f1 = f0 + kCycleSeg < sum ? f0 + kCycleSeg : sum;
-          for (uint64_t f = f0 + lane; f < f1; f += 32) {
-            while (off[j + 1] <= f) ++j;  // ends: off[CYC_THREADS] = sum > f
-            const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(ptr[j]) + (f - off[j]));
-            if (hash) {
-              local += HashBump(table, cnt, lg, w);
+          for (int t = 0; t < 4; ++t) {
+            if (f + 32 * t >= f1) break;
+            if (!TILED) {
+              local += HashBump(table, cnt, lg, w[t]);
             } else {
-              const uint32_t k = (uint32_t)(w - t0);
+              const uint32_t k = (uint32_t)(w[t] - t0);
               if (wide) {
                 local += atomicAdd(table + k, 1u);
               } else {
@@ -340,10 +360,10 @@ __global__ void __launch_bounds__(CYC_THREADS, 1) k_cycle4_cta(DGraph G, uint32_
             }
           }
         }
-        __syncthreads();  // the next chunk rewrites the offsets, the next range the table
       }
+      __syncthreads();  // the next chunk rewrites the offsets, the next root the table
     }
-    __syncthreads();  // s_item is rewritten
+    __syncthreads();  // s_item is rewritten (a root without candidates passes no barrier above)
   }
   local = WarpSum(local);
   if (lane == 0 && local) atomicAdd(acc, local);

@@ -2131,8 +2131,7 @@ class Executor {
       return false;
     if (prog_.form == C_CYCLE4) {
       if (Defects(true)) return false;
-      CountCycles(col, P);
-      return true;
+      return CountCycles(col, P);
     }
     const bool all = !task.list && task.begin == 0 && task.end >= g_.n && task.stride <= 1 && P == g_.n;
     const uint32_t bad = Defects(all && !oriented_);
@@ -2148,14 +2147,14 @@ class Executor {
 
   template <int K, bool ORIENT, int THREADS, bool GLOBAL>
   void LaunchCliqueClass(const CView& V, const uint32_t* col, const CliqueQueues& Q, int cls, uint32_t dmax,
-                         uint32_t* scratch) {
+                         uint32_t* scratch, cudaStream_t st) {
     const size_t smem = CliqueSmem(K, dmax, THREADS, GLOBAL);
     auto kernel = k_clique_cta<K, ORIENT, THREADS, GLOBAL>;
     // one attribute per instantiation and device (the largest class of it;
     // setting it twice from two threads is harmless)
     constexpr size_t kMost = GLOBAL       ? CliqueSmem(K, kCliqueG, THREADS, true)
-                             : THREADS == 128 ? CliqueSmem(K, kCliqueM, THREADS, false)
-                                              : CliqueSmem(K, CliqueX(K), THREADS, false);
+                             : THREADS == kCliqueMThreads ? CliqueSmem(K, kCliqueM, THREADS, false)
+                                                          : CliqueSmem(K, CliqueX(K), THREADS, false);
     static std::atomic<int> per_sm_of[64][2];  // resident CTAs: class L or the only one, class X
     const int dv = ctx_.device, slot = cls == 3 ? 1 : 0;
     int per_sm = dv >= 0 && dv < 64 ? per_sm_of[dv][slot].load(std::memory_order_acquire) : 0;
@@ -2166,7 +2165,7 @@ class Executor {
       if (dv >= 0 && dv < 64) per_sm_of[dv][slot].store(per_sm, std::memory_order_release);
     }
     const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sms_ * (GLOBAL ? 1 : per_sm), Q.cap[cls]);
-    kernel<<<grid, THREADS, smem, st_>>>(V, col, Q.q[cls], Q.n + cls, Q.cap[cls], Q.n + 8 + cls, dmax, scratch,
+    kernel<<<grid, THREADS, smem, st>>>(V, col, Q.q[cls], Q.n + cls, Q.cap[cls], Q.n + 8 + cls, dmax, scratch,
                                          ctrl_);
     Launched();
   }
@@ -2242,13 +2241,26 @@ class Executor {
       }
     }
     Timed t = TimerStart();
-    // heaviest classes first; a class no list can reach is not launched
-    if (Q.top == kCliqueG) LaunchCliqueClass<K, ORIENT, 256, true>(V, col, Q, 4, kCliqueG, scratch);
-    if (bound > kCliqueL) LaunchCliqueClass<K, ORIENT, 512, false>(V, col, Q, 3, CliqueX(K), nullptr);
-    if (bound > kCliqueM) LaunchCliqueClass<K, ORIENT, 512, false>(V, col, Q, 2, kCliqueL, nullptr);
-    if (bound > kCliqueS) LaunchCliqueClass<K, ORIENT, 128, false>(V, col, Q, 1, kCliqueM, nullptr);
+    // the classes are independent: the few large roots (first) run beside the
+    // many small ones on the context's second stream, so neither waits for the
+    // other's last CTAs; a class no list can reach is not launched
+    constexpr int kWide = K == 4 ? 1024 : 512;
+    const bool fork = bound > kCliqueM;
+    if (fork) {
+      CK(cudaEventRecord(ctx_.copy_ev[0], st_));
+      CK(cudaStreamWaitEvent(ctx_.copy_stream, ctx_.copy_ev[0], 0));
+      if (Q.top == kCliqueG)
+        LaunchCliqueClass<K, ORIENT, 256, true>(V, col, Q, 4, kCliqueG, scratch, ctx_.copy_stream);
+      if (bound > kCliqueL)
+        LaunchCliqueClass<K, ORIENT, kWide, false>(V, col, Q, 3, CliqueX(K), nullptr, ctx_.copy_stream);
+      LaunchCliqueClass<K, ORIENT, kWide, false>(V, col, Q, 2, kCliqueL, nullptr, ctx_.copy_stream);
+      CK(cudaEventRecord(ctx_.copy_ev[1], ctx_.copy_stream));
+    }
+    if (bound > kCliqueS)
+      LaunchCliqueClass<K, ORIENT, kCliqueMThreads, false>(V, col, Q, 1, kCliqueM, nullptr, st_);
     k_clique_small<K, ORIENT><<<WarpGrid(P), WARP_BLOCK, 0, st_>>>(V, col, Q.q[0], Q.n, Q.cap[0], ctrl_);
     Launched();
+    if (fork) CK(cudaStreamWaitEvent(st_, ctx_.copy_ev[1], 0));
     TimerStop(t, kPhaseComputeCount);
     if (left) {
       DFront F{};
@@ -2260,26 +2272,49 @@ class Executor {
     return true;
   }
 
-  void CountCycles(const uint32_t* col, uint32_t P) {
+  // 4-cycles through the roots col[0..P) by two-path counters (cycle.cuh).
+  bool CountCycles(const uint32_t* col, uint32_t P) {
+    // ranges of a root's counters, at most (the narrowest: 32-bit counters,
+    // which a graph of 65536 vertices or fewer never needs)
+    const uint64_t per = kCycleTable / (g_.n > 0xFFFFu ? 4 : 2);
+    const uint64_t ranges = (g_.n + per - 1) / per;
+    if (P * ranges > 0xFFFFFFFFull || P * (ranges * 8 + 4) > A_.Free() / 2) return false;
+    const size_t mark = A_.Mark();
     static std::atomic<bool> set[64];  // per device, once (twice is harmless)
     const int dv = ctx_.device;
     if (dv < 0 || dv >= 64 || !set[dv].load(std::memory_order_acquire)) {
       CK(cudaFuncSetAttribute(k_cycle4_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCycleWarpSmem));
-      CK(cudaFuncSetAttribute(k_cycle4_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCycleCtaSmem));
+      CK(cudaFuncSetAttribute(k_cycle4_cta<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCycleCtaSmem));
+      CK(cudaFuncSetAttribute(k_cycle4_cta<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCycleCtaSmem));
       if (dv >= 0 && dv < 64) set[dv].store(true, std::memory_order_release);
     }
-    uint32_t* ctl = (uint32_t*)A_.Alloc(4 * sizeof(uint32_t));  // next root, queued roots, next queued
+    // next root, queued roots, next queued, queued ranges, next range
+    uint32_t* ctl = (uint32_t*)A_.Alloc(8 * sizeof(uint32_t));
     uint32_t* queue = (uint32_t*)A_.Alloc((size_t)P * 4);
+    uint64_t* tiles = (uint64_t*)A_.Alloc((size_t)P * ranges * 8);
+    uint32_t* err = (uint32_t*)(ctrl_ + 3);
     const DGraph G = ViewOf(g_);
     paths_ += P;
     Timed t = TimerStart();
-    CK(cudaMemsetAsync(ctl, 0, 4 * sizeof(uint32_t), st_));
+    CK(cudaMemsetAsync(ctl, 0, 8 * sizeof(uint32_t), st_));
     const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sms_ * 2, (P + CYW_WARPS - 1) / CYW_WARPS);
+    const unsigned ctas = (unsigned)std::min<uint64_t>(sms_, P);
     k_cycle4_warp<<<grid, CYW_THREADS, kCycleWarpSmem, st_>>>(G, col, P, ctl, queue, ctl + 1, ctrl_);
-    k_cycle4_cta<<<(unsigned)std::min<uint64_t>(sms_, P), CYC_THREADS, kCycleCtaSmem, st_>>>(
-        G, (uint32_t)g_.n, col, queue, ctl + 1, ctl + 2, ctrl_);
-    TimerStop(t, kPhaseComputeCount);
+    k_cycle4_cta<false><<<ctas, CYC_THREADS, kCycleCtaSmem, st_>>>(G, (uint32_t)g_.n, col, queue, ctl + 1, ctl + 2,
+                                                                    tiles, ctl + 3, (uint32_t)(P * ranges), err,
+                                                                    ctrl_);
     launches_ += 2;
+    // more two-paths than the table takes need more than kCycleHashMax edges
+    if (g_.m > kCycleHashMax) {
+      const unsigned most = (unsigned)std::min<uint64_t>(sms_, (uint64_t)P * ranges);
+      k_cycle4_cta<true><<<most, CYC_THREADS, kCycleCtaSmem, st_>>>(G, (uint32_t)g_.n, col, queue, ctl + 1, ctl + 4,
+                                                                     tiles, ctl + 3, (uint32_t)(P * ranges), err,
+                                                                     ctrl_);
+      ++launches_;
+    }
+    TimerStop(t, kPhaseComputeCount);
+    A_.Release(mark);
+    return true;
   }
 
   // Loads, for the paths of Fb, the adjacency lists step `ds` intersects into
