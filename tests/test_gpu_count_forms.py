@@ -131,3 +131,38 @@ def test_cliques_of_skewed_graphs(resident):
         part = dict(root_begin=5, root_end=g.n - 9, root_stride=3)
         assert g.count(q, **part) == g.count(q, warp_granularity=3, **part)
         assert o.count(q, **part) == o.count(q, warp_granularity=2, **part)
+
+
+def test_batched_cycles_and_cliques():
+    # 4-cycles by counters (one range of w and several), cliques on oriented
+    # lists; graphs outside their contract, and oriented ones, as they are
+    graphs, queries = [], []
+
+    def add(g, *qs):
+        for q in qs:
+            graphs.append(g)
+            queries.append(q)
+
+    add(sme.Graph.er(64, 6.0, seed=1), 1, 0, 3)
+    add(sme.Graph.ba(700, 9, seed=2), 1, 0, 3, 7, 2)
+    add(sme.Graph.ba(4096, 6, seed=3), 1)
+    add(sme.Graph.ba(4097, 6, seed=4), 1, 3)
+    add(sme.Graph.rmat(14, 4, seed=5), 1, 0)
+    add(sme.Graph.clique(40), 1, 0, 3, 7, 11)
+    add(sme.Graph.clique(2), 1, 0, 3)
+    add(sme.Graph.rmat(10, 8, seed=6).degree_order(orient=True)[0], 0, 3, 7)
+    e = random_edges(300, 4000, 8)
+    add(sme.Graph.from_csr(*csr_of(300, e, both=False)), 1, 0, 3)
+    add(sme.Graph.from_csr(*csr_of(300, np.concatenate([e, [(4, 4)]]))), 1, 0)
+    hub = [(h, 2 + l) for h in range(2) for l in range(9000)]  # two hubs, three ranges
+    add(sme.Graph.from_csr(*csr_of(9002, hub)), 1)
+    want = [g.count(q, warp_granularity=1) if not g.oriented else g.count(q, warp_granularity=2)
+            for g, q in zip(graphs, queries)]
+    assert want[-1] == 9000 * 8999 // 2
+    # self loops: the batched plan checks every pair it orders, as before
+    for kw in (dict(), dict(autotune=False, granularity=1), dict(autotune=False, use_graph=False)):
+        plan = sme.BatchPlan(graphs, queries, **kw)
+        for _ in range(2):
+            assert plan.run()[0].tolist() == want, kw
+    only = sme.BatchPlan(graphs[:1], [1])  # nothing for the depth-first kernel
+    assert only.run()[0].tolist() == want[:1]
