@@ -55,40 +55,6 @@ __global__ void k_iota(uint32_t* out, uint32_t n, uint32_t start, uint32_t strid
     out[i] = start + i * stride;
 }
 
-// Children estimate of an intersection step: the smallest list (the pivot
-// size), an upper bound of the candidate count (ThreadEstimatePathCount<MIN>,
-// CheckConstraintsCommon.cuh:161-189).
-// With `sumdeg`, also the bytes of adjacency lists the path reads (external
-// mode: the subgraph a batch must load, EXTEstimateIntersectCost,
-// src/gpu/impl/light/ext/EXTLIGHTOrganizeBatch.cuh:11-53).
-__global__ void k_est_compute(DFront F, DStep s, const uintE* __restrict__ rp, uint64_t* est,
-                              uint64_t* sumdeg) {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < F.P; p += gridDim.x * blockDim.x) {
-    uint64_t m = ~0ULL, sd = 0;
-    for (int i = 0; i < s.nconn; ++i) {
-      uint32_t v = F.inst[s.conn[i]][p];
-      uint64_t d = rp[v + 1] - rp[v];
-      m = min(m, d);
-      sd += d;
-    }
-    if (sumdeg) sumdeg[p] = sd;
-    if (s.reuse >= 0) {
-      const uint32_t* ptr;
-      uint32_t len;
-      GetSet(F, s.reuse, p, ptr, len);
-      m = min(m, (uint64_t)len);
-    }
-    est[p] = m == ~0ULL ? 0 : m;
-  }
-}
-
-__global__ void k_est_set(DFront F, int u, uint64_t* est) {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < F.P; p += gridDim.x * blockDim.x) {
-    uint32_t s = SetIndex(F, u, p);
-    est[p] = F.set[u].cnt[s];
-  }
-}
-
 // ---- inclusive scan of uint64 (tile 4096 = 512 threads x 8) -------------
 constexpr int SCAN_THREADS = 512;
 constexpr int SCAN_ITEMS = 8;
@@ -121,6 +87,153 @@ __device__ uint64_t BlockExclusiveScan(uint64_t v, uint64_t* total) {
   if (total) *total = warp_tot[(blockDim.x >> 5) - 1];
   __syncthreads();
   return excl;
+}
+
+// What a scan sums per path:
+//   E_LIST  an intersection step's smallest list (the pivot size), an upper
+//           bound of the candidate count (ThreadEstimatePathCount<MIN>,
+//           CheckConstraintsCommon.cuh:161-189); with a second output, also
+//           the elements of the adjacency lists the path reads (external mode:
+//           what a batch must load, EXTEstimateIntersectCost,
+//           src/gpu/impl/light/ext/EXTLIGHTOrganizeBatch.cuh:11-53)
+//   E_SET   the size of u's candidate set
+//   E_CHILD the children of the path when u is materialised: the set's range
+//           clipped by < and >, minus the excluded values in it
+enum EstKind { E_LIST, E_SET, E_CHILD };
+
+template <EstKind KIND>
+__device__ __forceinline__ uint64_t EstOf(const DFront& F, const DStep& s, const DCond& c,
+                                          const uintE* __restrict__ rp, uint32_t p, uint64_t* lists) {
+  if (KIND == E_LIST) {
+    uint64_t m = ~0ULL, sd = 0;
+    for (int i = 0; i < s.nconn; ++i) {
+      const uint32_t v = F.inst[s.conn[i]][p];
+      const uint64_t d = __ldg(rp + v + 1) - __ldg(rp + v);
+      m = min(m, d);
+      sd += d;
+    }
+    *lists = sd;
+    if (s.reuse >= 0) {
+      const uint32_t* ptr;
+      uint32_t len;
+      GetSet(F, s.reuse, p, ptr, len);
+      m = min(m, (uint64_t)len);
+    }
+    return m == ~0ULL ? 0 : m;
+  }
+  const uint32_t* a;
+  uint32_t n;
+  GetSet(F, s.u, p, a, n);
+  if (KIND == E_SET) return n;
+  Bounds bd = MakeBounds(c, F, p);
+  uint32_t r0, r1, ex[MAXV];
+  Range(a, n, bd, r0, r1);
+  return (uint64_t)(r1 - r0 - Exclusions(a, r0, r1, bd, ex));
+}
+
+// Inclusive sums of the tile's estimates into `out` (and `out2`), the tile
+// sums into bs (bs2 = bs + nb + 1); the last block to finish turns the tile
+// sums into exclusive ones with the total after them.  One tile needs nothing
+// more; k_scan_add adds the tile sums otherwise.  The estimate, its scan and
+// the total were four launches and the host's split query before.  ITEMS 1
+// for frontiers of up to kScanSmall paths (an estimate is a chain of loads:
+// one per thread, over as many SMs as there are tiles), else SCAN_ITEMS.
+constexpr uint32_t kScanSmall = 148 * 4 * SCAN_THREADS;
+template <EstKind KIND, bool TWO, int ITEMS>
+__global__ void __launch_bounds__(SCAN_THREADS) k_est_scan(DFront F, DStep s, DCond c,
+                                                           const uintE* __restrict__ rp, uint64_t* out,
+                                                           uint64_t* out2, uint64_t* bs, uint32_t* ticket) {
+  const uint64_t base = (uint64_t)blockIdx.x * (SCAN_THREADS * ITEMS);
+  const uint32_t nb = gridDim.x;
+  uint64_t v[ITEMS], v2[TWO ? ITEMS : 1];
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    const uint64_t i = base + (uint64_t)k * SCAN_THREADS + threadIdx.x;
+    uint64_t lists = 0;
+    v[k] = i < F.P ? EstOf<KIND>(F, s, c, rp, (uint32_t)i, &lists) : 0;
+    if (TWO) v2[k] = lists;
+  }
+  uint64_t run = 0, run2 = 0;
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    const uint64_t i0 = base + (uint64_t)k * SCAN_THREADS;
+    if (i0 >= F.P) break;  // uniform in the block
+    const uint64_t i = i0 + threadIdx.x;
+    uint64_t total;
+    const uint64_t e = BlockExclusiveScan(v[k], &total);
+    if (i < F.P) out[i] = run + e + v[k];
+    run += total;
+    if (TWO) {
+      const uint64_t e2 = BlockExclusiveScan(v2[k], &total);
+      if (i < F.P) out2[i] = run2 + e2 + v2[k];
+      run2 += total;
+    }
+  }
+  uint64_t* bs2 = bs + nb + 1;
+  __shared__ uint32_t s_last;
+  if (threadIdx.x == 0) {
+    bs[blockIdx.x] = run;
+    if (TWO) bs2[blockIdx.x] = run2;
+    __threadfence();
+    s_last = atomicAdd(ticket, 1u) == nb - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();  // the other blocks' sums, read past L1
+  const uint32_t per = (nb + SCAN_THREADS - 1) / SCAN_THREADS;
+  for (int w = 0; w < (TWO ? 2 : 1); ++w) {
+    uint64_t* t = w ? bs2 : bs;
+    const uint32_t b = min(nb, threadIdx.x * per), e = min(nb, b + per);
+    uint64_t sum = 0, total;
+    for (uint32_t i = b; i < e; ++i) sum += __ldcg(t + i);
+    uint64_t at = BlockExclusiveScan(sum, &total);
+    for (uint32_t i = b; i < e; ++i) {
+      const uint64_t x = __ldcg(t + i);
+      t[i] = at;
+      at += x;
+    }
+    if (threadIdx.x == 0) t[nb] = total;
+  }
+  if (threadIdx.x == 0) *ticket = 0;  // for the next launch on the stream
+}
+
+template <bool TWO, int ITEMS>
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_add(uint64_t* out, uint64_t* out2, uint32_t n,
+                                                           const uint64_t* __restrict__ bs) {
+  const uint64_t base = (uint64_t)(blockIdx.x + 1) * (SCAN_THREADS * ITEMS);  // tile 0 stays as it is
+  const uint32_t nb = gridDim.x + 1;
+  const uint64_t add = bs[blockIdx.x + 1], add2 = TWO ? bs[nb + 1 + blockIdx.x + 1] : 0;
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    const uint64_t i = base + (uint64_t)k * SCAN_THREADS + threadIdx.x;
+    if (i < n) {
+      out[i] += add;
+      if (TWO) out2[i] += add2;
+    }
+  }
+}
+
+// ---- COMPUTE over one list: a view per path --------------------------------
+// The candidate set of a step that reads one list (or one earlier set) and has
+// no `!=` condition is a sub-range of it: one thread per path clips it; no
+// estimate, no scan and no data buffer.
+__global__ void __launch_bounds__(WARP_BLOCK) k_view(DFront F, DStep s, DGraph G, uint64_t* out_ptr,
+                                                     uint32_t* out_cnt, unsigned long long* acc) {
+  unsigned long long bytes = 0;
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < F.P; p += gridDim.x * blockDim.x) {
+    const uint32_t* a;
+    uint32_t n;
+    if (s.nconn) AdjList(G, F.inst[s.conn[0]][p], a, n);
+    else GetSet(F, s.reuse, p, a, n);
+    const BoundsT<0> bd = MakeBounds<0>(s.cond, F, p);
+    uint32_t r0, r1;
+    Range(a, n, bd, r0, r1);
+    out_ptr[p] = (uint64_t)(a + r0);
+    out_cnt[p] = r1 - r0;
+    bytes += 12ULL * s.nconn;
+  }
+  bytes = WarpSum(bytes);
+  if ((threadIdx.x & 31) == 0 && bytes) atomicAdd(acc + 1, bytes);
 }
 
 __global__ void k_scan_reduce(const uint64_t* __restrict__ in, uint32_t n, uint64_t* bs) {
@@ -196,12 +309,10 @@ __global__ void k_split(const uint64_t* __restrict__ incl, const uint64_t* __res
     if (c > t) hi = mid;
     else lo = mid + 1;
   }
-  out[2 * k] = lo;
-  out[2 * k + 1] = lo == 0 ? 0 : incl[lo - 1];
-  if (lo == start) {  // a single path above the budget: its own batch
-    out[2 * k] = start + 1;
-    out[2 * k + 1] = incl[start];
-  }
+  if (lo == start) ++lo;  // a single path above the budget: its own batch
+  out[3 * k] = lo;
+  out[3 * k + 1] = incl[lo - 1];  // lo > start >= 0
+  out[3 * k + 2] = incl2 ? incl2[lo - 1] : 0;
 }
 
 // ---- paths grouped by the hub they probe ------------------------------------
@@ -1046,20 +1157,6 @@ __global__ void __launch_bounds__(WARP_BLOCK, MINB) k_compute_flat(
 }
 
 // ---- MATERIALIZE ---------------------------------------------------------
-// Valid children per path: set range clipped by < / >, minus excluded values.
-__global__ void k_mat_count(DFront F, int u, DCond c, uint64_t* cnt) {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < F.P; p += gridDim.x * blockDim.x) {
-    const uint32_t* a;
-    uint32_t n;
-    GetSet(F, u, p, a, n);
-    Bounds bd = MakeBounds(c, F, p);
-    uint32_t r0, r1, ex[MAXV];
-    Range(a, n, bd, r0, r1);
-    int ne = Exclusions(a, r0, r1, bd, ex);
-    cnt[p] = (uint64_t)(r1 - r0 - ne);
-  }
-}
-
 // Expands each path's valid candidates into child rows: materialised columns
 // (broadcast from the parent) plus the new vertex, and the set index of every
 // live candidate set (Materialize, src/gpu/impl/light/op/LIGHTMaterialize.cuh:23-162,
@@ -1351,46 +1448,49 @@ __global__ void k_count_direct(DFront F, uint8_t nu, uint8_t u0, uint8_t u1, uin
 // scales with the vertex count except a start-over.
 constexpr uint64_t kAbsent = ~0ULL, kPending = ~0ULL - 1;
 
-__global__ void k_ext_claim(DFront F, DStep s, const uintE* __restrict__ rp, uint64_t* coff, uint32_t* newids,
-                            unsigned int* nnew) {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < F.P; p += gridDim.x * blockDim.x)
-    for (int i = 0; i < s.nconn; ++i) {
-      const uint32_t v = F.inst[s.conn[i]][p];
-      if (rp[v + 1] == rp[v] || coff[v] != kAbsent) continue;
-      if (atomicCAS(reinterpret_cast<unsigned long long*>(coff + v), kAbsent, kPending) == kAbsent)
-        newids[atomicAdd(nnew, 1u)] = v;
-    }
-}
-
-__global__ void k_ext_newdeg(const uint32_t* __restrict__ ids, uint32_t n, const uintE* __restrict__ rp,
-                             uint64_t* deg) {
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-    deg[k] = rp[ids[k] + 1] - rp[ids[k]];
-}
-
-__global__ void k_ext_place(const uint32_t* __restrict__ ids, uint32_t n, const uint64_t* __restrict__ deg_incl,
-                            uint64_t used, uint64_t* coff) {
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-    coff[ids[k]] = used + (k == 0 ? 0 : deg_incl[k - 1]);
-}
-
-// Copies the newly placed lists from pinned, mapped host memory into the
-// cache (one warp per list, coalesced reads over the host link); replaces
-// the host-thread gather + synchronous H2D of LoadSubgraph
-// (src/gpu/impl/common/ext/LoadSubgraph.h:10-42, EXTGraphGPUCommon.cuh:60-149).
-__global__ void __launch_bounds__(WARP_BLOCK) k_ext_gather(const uint32_t* __restrict__ ids, uint32_t nid,
-                                                           const uintE* __restrict__ rp,
-                                                           const uint32_t* __restrict__ host_cols,
-                                                           const uint64_t* __restrict__ coff,
-                                                           uint32_t* __restrict__ cache) {
+// Claims, places and gathers in one launch: a lane takes one list reference
+// of the batch, the lane that wins a missing list's claim places it after the
+// cache's last one, and the warp then copies the lists its lanes won from
+// pinned, mapped host memory (coalesced reads over the host link; replaces the
+// host-thread gather + synchronous H2D of LoadSubgraph,
+// src/gpu/impl/common/ext/LoadSubgraph.h:10-42, EXTGraphGPUCommon.cuh:60-149).
+// A list that does not fit raises `over` and stays pending; the host then
+// starts the cache over.
+__global__ void __launch_bounds__(WARP_BLOCK) k_ext_load(DFront F, DStep s, const uintE* __restrict__ rp,
+                                                         const uint32_t* __restrict__ host_cols, uint64_t* coff,
+                                                         uint32_t* __restrict__ cache, uint64_t cap,
+                                                         unsigned long long* used, unsigned long long* over) {
   const int lane = threadIdx.x & 31;
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t i = gw; i < nid; i += nw) {
-    const uint32_t v = ids[i];
-    const uintE b = rp[v], e = rp[v + 1];
-    const uint64_t o = coff[v];
-    for (uintE j = b + lane; j < e; j += 32) cache[o + (j - b)] = host_cols[j];
+  const uint64_t items = (uint64_t)F.P * s.nconn;
+  const uint64_t w0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull;
+  for (uint64_t b = w0; b < items; b += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t it = b + lane;
+    uint64_t from = 0, to = 0;
+    uint32_t len = 0;
+    if (it < items) {
+      const uint32_t v = F.inst[s.conn[it % s.nconn]][it / s.nconn];
+      const uint64_t r = __ldg(rp + v);
+      const uint32_t n = (uint32_t)(__ldg(rp + v + 1) - r);
+      if (n && __ldcg(coff + v) == kAbsent &&
+          atomicCAS(reinterpret_cast<unsigned long long*>(coff + v), kAbsent, kPending) == kAbsent) {
+        const uint64_t o = atomicAdd(used, (unsigned long long)n);
+        if (o + n <= cap) {
+          coff[v] = o;
+          from = r;
+          to = o;
+          len = n;
+        } else {
+          *over = 1;
+        }
+      }
+    }
+    for (unsigned won = __ballot_sync(FULL, len > 0); won; won &= won - 1) {
+      const int k = __ffs(won) - 1;
+      const uint32_t n = __shfl_sync(FULL, len, k);
+      const uint32_t* src = host_cols + __shfl_sync(FULL, (unsigned long long)from, k);
+      uint32_t* dst = cache + __shfl_sync(FULL, (unsigned long long)to, k);
+      for (uint32_t j = lane; j < n; j += 32) dst[j] = src[j];
+    }
   }
 }
 
@@ -1467,6 +1567,7 @@ void DestroyContext(DeviceContext* c) {
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
   for (auto e : c->copy_ev)
     if (e) cudaEventDestroy(e);
+  for (auto e : c->events) cudaEventDestroy(e);
   delete c;
 }
 
@@ -1988,6 +2089,8 @@ DStep ToDStep(const Step& s) {
   return d;
 }
 
+// Timing events a context keeps between runs.
+constexpr size_t kKeptEvents = 256;
 // Free arena below which every count runs its level program.
 constexpr uint64_t kFormArena = 64ULL << 20;
 
@@ -1996,6 +2099,13 @@ class Executor {
   Executor(const Program& prog, const DeviceGraph& g, DeviceContext& ctx, uint32_t* d_out, uint64_t cap)
       : prog_(prog), g_(g), ctx_(ctx), A_(ctx.arena), st_(ctx.stream), out_(d_out), cap_(cap) {
     sms_ = SmCount(ctx.device);
+  }
+
+  ~Executor() {
+    for (auto& e : events_) {
+      cudaEventDestroy(e.a);
+      cudaEventDestroy(e.b);
+    }
   }
 
   // External mode: adjacency lists are read from `host_cols` (pinned and
@@ -2012,9 +2122,7 @@ class Executor {
     A_.peak = mark;  // high-water mark of this run
     ctrl_ = (unsigned long long*)A_.Alloc(8 * sizeof(unsigned long long));
     if (ext_cols_) AllocExternalCache();
-    cudaEvent_t ev0, ev1;
-    CK(cudaEventCreate(&ev0));
-    CK(cudaEventCreate(&ev1));
+    const cudaEvent_t ev0 = TakeEvent(), ev1 = TakeEvent();
     CK(cudaEventRecord(ev0, st_));
     CK(cudaMemsetAsync(ctrl_, 0, 8 * sizeof(unsigned long long), st_));
     const Step& s0 = prog_.steps[0];
@@ -2048,8 +2156,6 @@ class Executor {
     CK(cudaStreamSynchronize(st_));
     float dev_ms = 0;
     cudaEventElapsedTime(&dev_ms, ev0, ev1);
-    cudaEventDestroy(ev0);
-    cudaEventDestroy(ev1);
     CK(cudaGetLastError());
     if (h[3])
       Fail(SME_ERR_CUDA, std::string(h[3] & ENGINE_ERR_BOUNDS ? "device bounds check failed" : "") +
@@ -2060,19 +2166,19 @@ class Executor {
     r.emitted = h[2];
     r.stats.algorithmic_bytes = h[1];
     r.stats.reuse_hits = h[5];
+    ext_bytes_ += h[6] * 4;
     r.stats.kernel_launches = launches_;
     r.stats.batches = batches_;
     r.stats.peak_device_bytes = A_.peak;
     r.stats.paths_processed = paths_;
-    double phase[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (auto& e : events_) {
-      float ms = 0;
-      cudaEventElapsedTime(&ms, e.a, e.b);
-      phase[e.phase] += ms;
-      cudaEventDestroy(e.a);
-      cudaEventDestroy(e.b);
+    HarvestTimers();
+    ctx_.events.push_back(ev0);
+    ctx_.events.push_back(ev1);
+    while (ctx_.events.size() > kKeptEvents) {
+      cudaEventDestroy(ctx_.events.back());
+      ctx_.events.pop_back();
     }
-    events_.clear();
+    const double* phase = phase_;
     for (int i = 0; i < 8; ++i) r.stats.phase_ms[i] = phase[i];
     // the intersection kernels: COMPUTE, COMPUTE_COUNT, COMPUTE_PATH_COUNT
     r.stats.kernel_ms = phase[kPhaseCompute] + phase[kPhaseComputeCount] + phase[kPhasePathCount];
@@ -2094,13 +2200,15 @@ class Executor {
   uint32_t* out_;
   uint64_t cap_;
   int sms_ = 148;
-  unsigned long long* ctrl_ = nullptr;  // [0] count [1] bytes [2] emitted [3] error flags [5] reuse hits
+  // [0] count [1] bytes [2] emitted [3] error flags [4] list cache overflow
+  // [5] reuse hits [6] list cache elements [7] ticket of k_est_scan
+  unsigned long long* ctrl_ = nullptr;
   uint64_t launches_ = 0, batches_ = 0, paths_ = 0, hot_ = 0, root_h2d_ = 0;
   const uint32_t* ext_cols_ = nullptr;
   uint64_t ext_bytes_ = 0;
   uint64_t* ext_off_ = nullptr;      // per vertex: list offset in the cache
   uint32_t* ext_cache_ = nullptr;    // device list cache
-  uint64_t ext_cap_ = 0, ext_used_ = 0, ext_restarts_ = 0;
+  uint64_t ext_cap_ = 0, ext_bound_ = 0;
 
   // The resident graph with its hub bitmaps (`use_bitmaps_` false: lists only).
   DGraph Resident() const {
@@ -2320,42 +2428,42 @@ class Executor {
   // Loads, for the paths of Fb, the adjacency lists step `ds` intersects into
   // a device subgraph allocated in the current arena frame (it stays valid
   // while deeper levels use candidate sets that point into it).
-  DGraph LoadSubgraph(const DFront& Fb, const DStep& ds) {
+  // `elems`: the elements of all those lists, counted per path.  What the
+  // cache holds is known here only as a bound (`ext_bound_`: the batches'
+  // elements since the last look); the device's own count is read when the
+  // bound no longer fits.
+  DGraph LoadSubgraph(const DFront& Fb, const DStep& ds, uint64_t elems) {
     if (!ext_cols_) return Resident();
     Timed tl = TimerStart();
-    const size_t mark = A_.Mark();
-    uint32_t* newids = (uint32_t*)A_.Alloc(std::max<size_t>((size_t)Fb.P * std::max<int>(ds.nconn, 1), 1) * 4);
-    unsigned int* nnew = (unsigned int*)A_.Alloc(sizeof(unsigned int));
-    uint64_t total = 0;
-    uint32_t K = 0;
-    for (int attempt = 0; attempt < 2; ++attempt) {
-      CK(cudaMemsetAsync(nnew, 0, sizeof(unsigned int), st_));
-      k_ext_claim<<<Grid(Fb.P, 256), 256, 0, st_>>>(Fb, ds, g_.row_ptrs, ext_off_, newids, nnew);
+    unsigned long long* used = ctrl_ + 6;
+    unsigned long long* over = ctrl_ + 4;
+    auto load = [&] {
+      k_ext_load<<<Grid((uint64_t)Fb.P * std::max<int>(ds.nconn, 1), WARP_BLOCK), WARP_BLOCK, 0, st_>>>(
+          Fb, ds, g_.row_ptrs, ext_cols_, ext_off_, ext_cache_, ext_cap_, used, over);
       Launched();
-      K = (uint32_t)ReadU32(nnew);
-      if (K == 0) break;
-      uint64_t* deg = (uint64_t*)A_.Alloc((size_t)K * 8);
-      k_ext_newdeg<<<Grid(K, 256), 256, 0, st_>>>(newids, K, g_.row_ptrs, deg);
-      Launched();
-      Scan(deg, K);
-      total = ReadU64(deg + K - 1);
-      if (ext_used_ + total <= ext_cap_) {
-        k_ext_place<<<Grid(K, 256), 256, 0, st_>>>(newids, K, deg, ext_used_, ext_off_);
-        k_ext_gather<<<WarpGrid(K), WARP_BLOCK, 0, st_>>>(newids, K, g_.row_ptrs, ext_cols_, ext_off_, ext_cache_);
-        launches_ += 2;
-        ext_used_ += total;
-        ext_bytes_ += total * 4;
-        break;
-      }
-      if (attempt == 1)
-        Fail(SME_ERR_OOM, "external mode: the lists one batch reads (" + std::to_string(total * 4) +
-                              " bytes) exceed the device list cache (" + std::to_string(ext_cap_ * 4) + " bytes)");
+    };
+    if (ext_bound_ + elems > ext_cap_) ext_bound_ = ReadU64((const uint64_t*)used);
+    load();
+    if (ext_bound_ + elems <= ext_cap_) {
+      ext_bound_ += elems;
+    } else if (ReadU64((const uint64_t*)over) == 0) {  // lists the cache held already made room
+      ext_bound_ = ReadU64((const uint64_t*)used);
+    } else {
       // the cache is full: start over with this batch's lists
+      ext_bytes_ += std::min<uint64_t>(ReadU64((const uint64_t*)used), ext_cap_) * 4;
       CK(cudaMemsetAsync(ext_off_, 0xff, (size_t)(g_.n + 1) * 8, st_));
-      ext_used_ = 0;
-      ++ext_restarts_;
+      CK(cudaMemsetAsync(used, 0, 8, st_));
+      CK(cudaMemsetAsync(over, 0, 8, st_));
+      load();
+      ext_bound_ = elems;
+      if (elems > ext_cap_) {
+        if (ReadU64((const uint64_t*)over))
+          Fail(SME_ERR_OOM, "external mode: the lists one batch reads (" +
+                                std::to_string(ReadU64((const uint64_t*)used) * 4) +
+                                " bytes) exceed the device list cache (" + std::to_string(ext_cap_ * 4) + " bytes)");
+        ext_bound_ = ReadU64((const uint64_t*)used);
+      }
     }
-    A_.Release(mark);
     TimerStop(tl, kPhaseExternal);
     return DGraph{g_.row_ptrs, ext_cache_, nullptr, nullptr, 0, ext_off_, nullptr, 0};
   }
@@ -2374,7 +2482,7 @@ class Executor {
     const uint64_t bytes = std::max<uint64_t>(A_.Free() / 2, 1 << 20) & ~uint64_t(255);
     ext_cache_ = (uint32_t*)A_.Alloc(bytes);
     ext_cap_ = bytes / 4;
-    ext_used_ = 0;
+    ext_bound_ = 0;
   }
 
   // Batch cost of an external step in frontier-budget units: the subgraph
@@ -2383,7 +2491,8 @@ class Executor {
   double ExtListCost(uint64_t budget) const {
     return ext_cols_ && ext_cap_ ? 4.0 * (double)std::max<uint64_t>(budget, 1 << 20) / (double)(ext_cap_ * 4) : 0.0;
   }
-  std::vector<Timed> events_;
+  std::vector<Timed> events_;  // recorded regions
+  double phase_[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 
   void Launched() { ++launches_; }
 
@@ -2618,10 +2727,33 @@ class Executor {
     return (uint64_t)((double)A_.Free() * 0.85 / (double)rem);
   }
 
+  // Timing events come from the context's free list and go back to it.
+  cudaEvent_t TakeEvent() {
+    if (!ctx_.events.empty()) {
+      cudaEvent_t e = ctx_.events.back();
+      ctx_.events.pop_back();
+      return e;
+    }
+    cudaEvent_t e = nullptr;
+    CK(cudaEventCreate(&e));
+    return e;
+  }
+  // Adds the finished regions to their phases (the stream has passed them).
+  void HarvestTimers() {
+    for (auto& e : events_) {
+      float ms = 0;
+      cudaEventElapsedTime(&ms, e.a, e.b);
+      phase_[e.phase] += ms;
+      ctx_.events.push_back(e.a);
+      ctx_.events.push_back(e.b);
+    }
+    events_.clear();
+  }
+
   Timed TimerStart() {
     Timed e;
-    cudaEventCreate(&e.a);
-    cudaEventCreate(&e.b);
+    e.a = TakeEvent();
+    e.b = TakeEvent();
     cudaEventRecord(e.a, st_);
     e.phase = 0;
     return e;
@@ -2655,31 +2787,76 @@ class Executor {
   struct Batch {
     uint32_t b0, b1;
     uint64_t e0, e1;  // inclusive estimate before b0 / at b1-1
+    uint64_t lists;   // external mode: elements of the lists its paths read
   };
+
+  // Inclusive sums of a step's estimates over the paths into `est` (external
+  // mode: of its list elements into `est2`), and their totals.
+  struct Totals {
+    uint64_t est, lists;
+  };
+  template <EstKind KIND, int ITEMS>
+  void LaunchEstScan(const DFront& F, const DStep& ds, const DCond& dc, uint64_t* est, uint64_t* est2, uint32_t nb,
+                     uint64_t* bs) {
+    uint32_t* ticket = (uint32_t*)(ctrl_ + 7);
+    if (est2)
+      k_est_scan<E_LIST, true, ITEMS><<<nb, SCAN_THREADS, 0, st_>>>(F, ds, dc, g_.row_ptrs, est, est2, bs, ticket);
+    else
+      k_est_scan<KIND, false, ITEMS><<<nb, SCAN_THREADS, 0, st_>>>(F, ds, dc, g_.row_ptrs, est, nullptr, bs, ticket);
+    Launched();
+    if (nb == 1) return;
+    if (est2) k_scan_add<true, ITEMS><<<nb - 1, SCAN_THREADS, 0, st_>>>(est, est2, F.P, bs);
+    else k_scan_add<false, ITEMS><<<nb - 1, SCAN_THREADS, 0, st_>>>(est, nullptr, F.P, bs);
+    Launched();
+  }
+  template <EstKind KIND>
+  Totals EstScan(const DFront& F, const DStep& ds, const DCond& dc, uint64_t* est, uint64_t* est2) {
+    const uint32_t tile = F.P <= kScanSmall ? SCAN_THREADS : SCAN_TILE;
+    const uint32_t nb = (F.P + tile - 1) / tile;
+    const size_t m = A_.Mark();
+    uint64_t* bs = (uint64_t*)A_.Alloc(((size_t)nb + 1) * 16);
+    if (tile == SCAN_THREADS) LaunchEstScan<KIND, 1>(F, ds, dc, est, est2, nb, bs);
+    else LaunchEstScan<KIND, SCAN_ITEMS>(F, ds, dc, est, est2, nb, bs);
+    CK(cudaMemcpyAsync(ctx_.h_pinned, bs + nb, 8, cudaMemcpyDeviceToHost, st_));
+    if (est2) CK(cudaMemcpyAsync(ctx_.h_pinned + 1, bs + 2 * nb + 1, 8, cudaMemcpyDeviceToHost, st_));
+    CK(cudaStreamSynchronize(st_));
+    if (events_.size() >= kKeptEvents / 2) HarvestTimers();
+    A_.Release(m);
+    return Totals{ctx_.h_pinned[0], est2 ? ctx_.h_pinned[1] : 0};
+  }
+
+  // The batches of P paths: one when the whole cost fits the budget, else cut
+  // on the device.
+  std::vector<Batch> Batches(const uint64_t* incl, uint32_t P, double pf, double cf, uint64_t budget, Totals t,
+                             const uint64_t* incl2 = nullptr, double cg = 0) {
+    budget = std::max<uint64_t>(budget, 1 << 20);
+    if (pf * P + cf * (double)t.est + cg * (double)t.lists <= (double)budget)
+      return {Batch{0, P, 0, t.est, t.lists}};
+    return Split(incl, P, pf, cf, budget, incl2, cg);
+  }
 
   std::vector<Batch> Split(const uint64_t* incl, uint32_t P, double pf, double cf, uint64_t budget,
                            const uint64_t* incl2 = nullptr, double cg = 0) {
     std::vector<Batch> out;
     if (P == 0) return out;
-    budget = std::max<uint64_t>(budget, 1 << 20);
-    const uint32_t K = (uint32_t)std::min<size_t>(ctx_.pinned_words / 2, 4096);
+    const uint32_t K = (uint32_t)std::min<size_t>(ctx_.pinned_words / 3, (64 << 10) / 24);
     size_t m = A_.Mark();
-    uint64_t* d = (uint64_t*)A_.Alloc((size_t)K * 16);
+    uint64_t* d = (uint64_t*)A_.Alloc((size_t)K * 24);
     uint32_t start = 0;
-    uint64_t e_start = 0;
+    uint64_t e_start = 0, l_start = 0;
     while (start < P) {
       k_split<<<(K + 255) / 256, 256, 0, st_>>>(incl, incl2, P, start, pf, cf, cg, (double)budget, K, d);
       Launched();
-      CK(cudaMemcpyAsync(ctx_.h_pinned, d, (size_t)K * 16, cudaMemcpyDeviceToHost, st_));
+      CK(cudaMemcpyAsync(ctx_.h_pinned, d, (size_t)K * 24, cudaMemcpyDeviceToHost, st_));
       CK(cudaStreamSynchronize(st_));
       const uint64_t* h = ctx_.h_pinned;
       for (uint32_t k = 0; k < K && start < P; ++k) {
-        uint32_t end = (uint32_t)std::min<uint64_t>(h[2 * k], P);
+        uint32_t end = (uint32_t)std::min<uint64_t>(h[3 * k], P);
         if (end <= start) continue;
-        uint64_t e_end = h[2 * k + 1];
-        out.push_back(Batch{start, end, e_start, e_end});
+        out.push_back(Batch{start, end, e_start, h[3 * k + 1], h[3 * k + 2] - l_start});
         start = end;
-        e_start = e_end;
+        e_start = h[3 * k + 1];
+        l_start = h[3 * k + 2];
       }
     }
     A_.Release(m);
@@ -2703,6 +2880,53 @@ class Executor {
     k_emit<<<Grid(F.P, 256), 256, 0, st_>>>(F, (uint8_t)prog_.n, nullptr, sl[0], sl[1], sl[2], sl[3],
                                             sl[4], sl[5], out_, cap_, ctrl_ + 2);
     Launched();
+  }
+
+  void View(const DFront& F, const DStep& ds, const DGraph& G, uint64_t* ptr, uint32_t* cnt) {
+    Timed t = TimerStart();
+    k_view<<<Grid(F.P, WARP_BLOCK), WARP_BLOCK, 0, st_>>>(F, ds, G, ptr, cnt, ctrl_);
+    TimerStop(t, kPhaseCompute);
+    Launched();
+  }
+
+  // Expands the paths of F into their C children (`cnt`: inclusive child
+  // counts) and runs the next level on them.
+  void Materialize(size_t k, const DFront& F, const DCond& dc, const uint64_t* cnt, uint64_t C) {
+    if (C == 0) return;
+    if (C > 0x7fffffffULL) Fail(SME_ERR_OOM, "materialised batch exceeds 2^31 partial instances");
+    const Step& s = prog_.steps[k];
+    uint32_t* err = (uint32_t*)(ctrl_ + 3);
+    DMatOut o{};
+    o.u = s.u;
+    o.keep = s.keep_set;
+    o.nmat = (uint8_t)s.mat_after.size();
+    for (size_t i = 0; i < s.mat_after.size(); ++i) {
+      o.mat[i] = s.mat_after[i];
+      o.inst[s.mat_after[i]] = (uint32_t*)A_.Alloc(C * 4);
+    }
+    o.nsets = (uint8_t)s.sets_after.size();
+    for (size_t i = 0; i < s.sets_after.size(); ++i) {
+      o.sets[i] = s.sets_after[i];
+      o.cidx[s.sets_after[i]] = (uint32_t*)A_.Alloc(C * 4);
+    }
+    Timed tm = TimerStart();
+    k_mat_write<<<WarpGrid(F.P), WARP_BLOCK, 0, st_>>>(F, dc, o, cnt, C, kMatBig, err);
+    Launched();
+    if (C > kMatBig) {  // else no parent has more
+      k_mat_write_big<<<WarpGrid((C + kMatChunk - 1) / kMatChunk), WARP_BLOCK, 0, st_>>>(F, dc, o, cnt, C, kMatBig,
+                                                                                         err);
+      Launched();
+    }
+    TimerStop(tm, kPhaseMaterialize);
+    DFront Fn{};
+    Fn.P = (uint32_t)C;
+    for (int v = 0; v < MAXV; ++v) Fn.inst[v] = o.inst[v];
+    for (uint8_t w : s.sets_after) {
+      Fn.set[w] = F.set[w];
+      Fn.nset[w] = F.nset[w];
+      Fn.cidx[w] = o.cidx[w];
+    }
+    Level(k + 1, Fn);
   }
 
   void Level(size_t k, const DFront& F) {
@@ -2730,16 +2954,15 @@ class Executor {
         const size_t m0 = A_.Mark();
         uint64_t* est = (uint64_t*)A_.Alloc((size_t)F.P * 8);
         uint64_t* sd = (uint64_t*)A_.Alloc((size_t)F.P * 8);
-        k_est_compute<<<Grid(F.P, 256), 256, 0, st_>>>(F, ds, g_.row_ptrs, est, sd);
-        Launched();
-        Scan(sd, F.P);
+        const Totals tot = EstScan<E_LIST>(F, ds, DCond{}, est, sd);
         const uint64_t bk = Budget(k);
-        std::vector<Batch> bs = Split(sd, F.P, 12.0, 0.0, bk, sd, ExtListCost(bk));
+        const std::vector<Batch> bs =
+            Batches(sd, F.P, 12.0, 0.0, bk, Totals{tot.lists, tot.lists}, sd, ExtListCost(bk));
         for (const Batch& b : bs) {
           const size_t mk = A_.Mark();
           DFront Fb = Slice(F, b.b0, b.b1);
           ++batches_;
-          DGraph gv = LoadSubgraph(Fb, ds);
+          DGraph gv = LoadSubgraph(Fb, ds, b.lists);
           Compute<1>(Fb, ds, gv, nullptr, 0, nullptr, nullptr, nullptr, 0);
           A_.Release(mk);
         }
@@ -2776,33 +2999,52 @@ class Executor {
         break;
     }
     const size_t mark0 = A_.Mark();
-    uint64_t* est = (uint64_t*)A_.Alloc((size_t)F.P * 8);
-    uint64_t* sumdeg = nullptr;  // external mode: subgraph bytes per path
-    double pf = 0, cf = 0;
-    Timed to = TimerStart();
-    if (s.kind == S_COMPUTE || s.kind == S_PATH_COUNT) {
-      if (ext_cols_) sumdeg = (uint64_t*)A_.Alloc((size_t)F.P * 8);
-      k_est_compute<<<Grid(F.P, 256), 256, 0, st_>>>(F, ds, g_.row_ptrs, est, sumdeg);
-      pf = 12 + 16;
-      cf = s.kind == S_COMPUTE ? 4 : 0;
-    } else {  // MATERIALIZE, FILTER
-      k_est_set<<<Grid(F.P, 256), 256, 0, st_>>>(F, s.u, est);
-      if (s.kind == S_FILTER) {
-        pf = 12 + 16;
-        cf = 4;
-      } else {
-        pf = 16;
-        cf = 4.0 * (s.mat_after.size() + s.sets_after.size()) + 16;
+    const DCond dc = ToDCond(s.cond);
+    bool has_ne = false;
+    for (int i = 0; i < dc.n; ++i) has_ne |= dc.op[i] == 2;
+    uint64_t* est = nullptr;
+    uint64_t* sumdeg = nullptr;  // external mode: list elements per path
+    std::vector<Batch> batches;
+    // a step over one list without `!=` writes views, a path count nothing but
+    // counts: when one batch holds them there is nothing to estimate
+    const bool view = s.kind == S_COMPUTE && !ext_cols_ && ds.msrc < 0 && ds.nconn + (ds.reuse >= 0 ? 1 : 0) == 1 &&
+                      !has_ne && (gran_ == 0 || gran_ == 2);
+    const double fixed = 12 + 16;  // estimate, pointer and count per path
+    if ((view || (s.kind == S_PATH_COUNT && !ext_cols_)) && fixed * F.P <= (double)Budget(k)) {
+      batches.push_back(Batch{0, F.P, 0, 0, 0});
+    } else if (s.kind == S_MATERIALIZE) {
+      // one batch when all children fit, counted exactly; else batches by the
+      // set sizes, an upper bound, each counted in its turn
+      Timed to = TimerStart();
+      uint64_t* cnt = (uint64_t*)A_.Alloc((size_t)F.P * 8);
+      const Totals t = EstScan<E_CHILD>(F, ds, dc, cnt, nullptr);
+      TimerStop(to, kPhaseOrganize);
+      const double pf = 16, cf = 4.0 * (s.mat_after.size() + s.sets_after.size()) + 16;
+      if (pf * F.P + cf * (double)t.est <= (double)Budget(k) && t.est <= 2000000000ull) {
+        ++batches_;
+        Materialize(k, F, dc, cnt, t.est);
+        A_.Release(mark0);
+        return;
       }
+      A_.Release(mark0);
+      est = (uint64_t*)A_.Alloc((size_t)F.P * 8);
+      to = TimerStart();
+      EstScan<E_SET>(F, ds, dc, est, nullptr);
+      TimerStop(to, kPhaseOrganize);
+      // child counts of a batch stay within 31-bit path indices
+      const uint64_t bk = std::min<uint64_t>(Budget(k), (uint64_t)(cf * 2.0e9));
+      batches = Split(est, F.P, pf, cf, std::max<uint64_t>(bk, 1 << 20));
+    } else {  // COMPUTE, PATH_COUNT, FILTER
+      Timed to = TimerStart();
+      est = (uint64_t*)A_.Alloc((size_t)F.P * 8);
+      if (ext_cols_ && s.kind != S_FILTER) sumdeg = (uint64_t*)A_.Alloc((size_t)F.P * 8);
+      const Totals t = s.kind == S_FILTER ? EstScan<E_SET>(F, ds, dc, est, nullptr)
+                                          : EstScan<E_LIST>(F, ds, dc, est, sumdeg);
+      TimerStop(to, kPhaseOrganize);
+      const double cf = s.kind == S_PATH_COUNT ? 0 : 4;
+      const uint64_t bk = std::min<uint64_t>(Budget(k), (uint64_t)(std::max(cf, 1.0) * 2.0e9));
+      batches = Batches(est, F.P, fixed, cf, bk, t, sumdeg, ExtListCost(bk));
     }
-    Launched();
-    Scan(est, F.P);
-    if (sumdeg) Scan(sumdeg, F.P);
-    TimerStop(to, kPhaseOrganize);
-    uint64_t budget = Budget(k);
-    // keep child counts of a batch within 31-bit path indices
-    budget = std::min<uint64_t>(budget, (uint64_t)(std::max(cf, 1.0) * 2.0e9));
-    std::vector<Batch> batches = Split(est, F.P, pf, cf, budget, sumdeg, ExtListCost(budget));
     for (const Batch& b : batches) {
       const size_t mark = A_.Mark();
       DFront Fb = Slice(F, b.b0, b.b1);
@@ -2814,10 +3056,12 @@ class Executor {
           paths_ += Pb;
           uint64_t* ptr = (uint64_t*)A_.Alloc((size_t)Pb * 8);
           uint32_t* cnt = (uint32_t*)A_.Alloc((size_t)Pb * 4);
-          uint64_t cap = s.kind == S_COMPUTE ? b.e1 - b.e0 : 0;
+          uint64_t cap = s.kind == S_COMPUTE && !view ? b.e1 - b.e0 : 0;
           uint32_t* data = cap ? (uint32_t*)A_.Alloc(cap * 4) : nullptr;
-          DGraph gv = LoadSubgraph(Fb, ds);
-          if (s.kind == S_COMPUTE)
+          DGraph gv = LoadSubgraph(Fb, ds, b.lists);
+          if (view)
+            View(Fb, ds, gv, ptr, cnt);
+          else if (s.kind == S_COMPUTE)
             Compute<0>(Fb, ds, gv, est, b.b0, ptr, cnt, data, cap);
           else
             Compute<2>(Fb, ds, gv, est, b.b0, ptr, cnt, nullptr, 0);
@@ -2848,43 +3092,11 @@ class Executor {
           break;
         }
         case S_MATERIALIZE: {
-          DCond dc = ToDCond(s.cond);
           uint64_t* cnt = (uint64_t*)A_.Alloc((size_t)Pb * 8);
           Timed tm = TimerStart();
-          k_mat_count<<<Grid(Pb, 256), 256, 0, st_>>>(Fb, s.u, dc, cnt);
-          Launched();
-          Scan(cnt, Pb);
-          uint64_t C = ReadU64(cnt + Pb - 1);
-          if (C == 0) break;
-          if (C > 0x7fffffffULL) Fail(SME_ERR_OOM, "materialised batch exceeds 2^31 partial instances");
-          DMatOut o{};
-          o.u = s.u;
-          o.keep = s.keep_set;
-          o.nmat = (uint8_t)s.mat_after.size();
-          for (size_t i = 0; i < s.mat_after.size(); ++i) {
-            o.mat[i] = s.mat_after[i];
-            o.inst[s.mat_after[i]] = (uint32_t*)A_.Alloc(C * 4);
-          }
-          o.nsets = (uint8_t)s.sets_after.size();
-          for (size_t i = 0; i < s.sets_after.size(); ++i) {
-            o.sets[i] = s.sets_after[i];
-            o.cidx[s.sets_after[i]] = (uint32_t*)A_.Alloc(C * 4);
-          }
-          k_mat_write<<<WarpGrid(Pb), WARP_BLOCK, 0, st_>>>(Fb, dc, o, cnt, C, kMatBig, err);
-          k_mat_write_big<<<WarpGrid((C + kMatChunk - 1) / kMatChunk), WARP_BLOCK, 0, st_>>>(Fb, dc, o, cnt, C,
-                                                                                             kMatBig, err);
-          Launched();
+          const uint64_t C = EstScan<E_CHILD>(Fb, ds, dc, cnt, nullptr).est;
           TimerStop(tm, kPhaseMaterialize);
-          Launched();
-          DFront Fn{};
-          Fn.P = (uint32_t)C;
-          for (int v = 0; v < MAXV; ++v) Fn.inst[v] = o.inst[v];
-          for (uint8_t w : s.sets_after) {
-            Fn.set[w] = Fb.set[w];
-            Fn.nset[w] = Fb.nset[w];
-            Fn.cidx[w] = o.cidx[w];
-          }
-          Level(k + 1, Fn);
+          Materialize(k, Fb, dc, cnt, C);
           break;
         }
         default:

@@ -49,6 +49,7 @@ struct DeviceContext {
   cudaStream_t stream = nullptr;
   cudaStream_t copy_stream = nullptr;             // per-call uploads
   cudaEvent_t copy_ev[kUploadChunks + 1] = {};    // upload ranges landed
+  std::vector<cudaEvent_t> events;                // free timing events
   Arena arena;
   uint64_t* h_pinned = nullptr;  // small pinned host buffer for batch bounds
   size_t pinned_words = 0;
