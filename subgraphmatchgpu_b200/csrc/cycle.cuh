@@ -29,7 +29,6 @@ namespace dev {
 // bit 1 (sym): some v in N(u) has no u in N(v).  Warps take chunks of
 // consecutive edges, so a hub's list is spread over many warps.
 constexpr uint32_t kNotSimple = 1u, kNotSymmetric = 2u;
-constexpr uint32_t kCheckChunk = 512;
 
 // Last u in [0, n) with rp[u] <= e (the owner of edge e), by the whole warp.
 __device__ __forceinline__ uint32_t WarpOwner(const uint64_t* __restrict__ rp, uint32_t n, uint64_t e) {
@@ -52,13 +51,14 @@ __device__ __forceinline__ uint32_t WarpOwner(const uint64_t* __restrict__ rp, u
 }
 
 template <bool SYM>
-__global__ void __launch_bounds__(WARP_BLOCK) k_check_simple(DGraph G, uint32_t n, uint64_t m, uint32_t* flag) {
+__global__ void __launch_bounds__(WARP_BLOCK) k_check_simple(DGraph G, uint32_t n, uint64_t m, uint32_t chunk,
+                                                             uint32_t* flag) {
   const int lane = threadIdx.x & 31;
   const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   uint32_t bad = 0;
-  for (uint64_t c0 = gw * kCheckChunk; c0 < m; c0 += nw * kCheckChunk) {
-    const uint64_t c1 = c0 + kCheckChunk < m ? c0 + kCheckChunk : m;
+  for (uint64_t c0 = gw * chunk; c0 < m; c0 += nw * chunk) {
+    const uint64_t c1 = c0 + chunk < m ? c0 + chunk : m;
     uint32_t u = WarpOwner(G.rp, n, c0);
     for (uint64_t e = c0 + lane; e < c1; e += 32) {
       while (__ldg(G.rp + u + 1) <= e) ++u;  // ends: rp[n] = m > e
