@@ -535,15 +535,41 @@ static void RequireSiblingLayout(Program& p) {
 // Counts with a kernel of their own, under every plan (the number does not
 // depend on it), while the options ask for nothing about how the steps run: an
 // explicit launch shape, lists without bitmaps, a plan variant or external
-// mode keep the level program.  The root of the task must be pattern vertex 0.
+// mode keep the level program.  The root of the task must be pattern vertex 0
+// (the house's: vertex 1, as in the LIGHT plan).
 static CountForm FormOf(const sme_opts& o, const Query& q, const Program& p, bool enumerate) {
   if (enumerate || !q.enable_ordering || o.execute_mode != SME_IN_MEMORY_GPU || o.warp_granularity != 0 ||
       o.list_only || o.no_set_reuse || o.reuse_autogen >= 0 || o.compress_level != SME_COMPRESS_SPECIAL ||
-      p.steps[0].kind != S_INIT || p.out_slot[p.steps[0].u] != 0)
+      p.steps[0].kind != S_INIT)
     return C_STEPS;
+  const int root = p.out_slot[p.steps[0].u];
+  if (q.type == 4 && root == 1) return C_HOUSE;
+  if (root != 0) return C_STEPS;
   if (q.type == 1) return C_CYCLE4;
   if (q.n >= 4 && IsOrderedClique(q)) return C_CLIQUE;
   return C_STEPS;
+}
+
+// The triangles (u1, u2, u0) of the house with u1 < u2 and, per triangle, the
+// common neighbours of u2 and u0 (house.cuh).
+static std::vector<Step> HouseMinus() {
+  std::vector<Step> steps(6);
+  auto set = [&](int i, StepKind k, uint8_t u, std::vector<uint8_t> conn, std::vector<uint8_t> mat,
+                 std::vector<uint8_t> sets) {
+    steps[i].kind = k;
+    steps[i].u = u;
+    steps[i].conn = conn;
+    steps[i].mat_after = mat;
+    steps[i].sets_after = sets;
+  };
+  set(0, S_INIT, 1, {}, {1}, {});
+  set(1, S_COMPUTE, 2, {1}, {1}, {2});
+  steps[1].cond.push_back(StepCond{LARGER_THAN, 1});
+  set(2, S_MATERIALIZE, 2, {}, {1, 2}, {});
+  set(3, S_COMPUTE, 0, {1, 2}, {1, 2}, {0});
+  set(4, S_MATERIALIZE, 0, {}, {2, 0}, {});
+  set(5, S_COMPUTE_COUNT, 4, {2, 0}, {2, 0}, {});
+  return steps;
 }
 
 Program Compile(const sme_opts& o, bool enumerate, bool loop_free) {
@@ -573,6 +599,7 @@ Program Compile(const sme_opts& o, bool enumerate, bool loop_free) {
   RequireSiblingLayout(p);
   if (!enumerate) AliasRepeatedComputes(p);
   p.form = FormOf(o, q, p, enumerate);
+  if (p.form == C_HOUSE) p.minus = HouseMinus();
   for (auto& s : p.steps) {
     std::ostringstream os;
     os << KindName(s.kind) << "(" << (int)s.u << ")";

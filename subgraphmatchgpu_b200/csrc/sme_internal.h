@@ -243,7 +243,8 @@ struct Step {
 enum CountForm : uint8_t {
   C_STEPS = 0,   // the level program
   C_CYCLE4 = 1,  // Q1: two-path counters (cycle.cuh)
-  C_CLIQUE = 2   // Q3, Q7, Q11: bit matrices per root (clique.cuh)
+  C_CLIQUE = 2,  // Q3, Q7, Q11: bit matrices per root (clique.cuh)
+  C_HOUSE = 3    // Q4 rooted at u1: two-path counters (house.cuh) less `minus`
 };
 struct Program {
   CountForm form = C_STEPS;
@@ -251,6 +252,9 @@ struct Program {
   int n = 0;               // pattern vertices
   int algo = SME_GPU_LIGHT;
   std::vector<Step> steps;
+  // C_HOUSE: the level program whose count, less its last step's paths, is
+  // subtracted from the counters' sum
+  std::vector<Step> minus;
   std::vector<uint8_t> out_slot;  // plan vertex -> tuple position
   bool enumerate = false;
   std::string Describe() const;

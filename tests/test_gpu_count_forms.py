@@ -166,3 +166,37 @@ def test_batched_cycles_and_cliques():
             assert plan.run()[0].tolist() == want, kw
     only = sme.BatchPlan(graphs[:1], [1])  # nothing for the depth-first kernel
     assert only.run()[0].tolist() == want[:1]
+
+
+@pytest.mark.parametrize("n", [5, 12, 20, 65, 130])
+def test_houses_of_complete_graphs(n):
+    g = sme.Graph.clique(n)
+    g.to_device(0)
+    assert g.count(4) == 60 * comb(n, 5)  # 5! placements, two of them alike
+
+
+@pytest.mark.parametrize("scale,ef,seed", [(9, 8, 1), (11, 6, 2), (12, 8, 3)])
+def test_houses_match_the_level_program(scale, ef, seed):
+    g = sme.Graph.rmat(scale, ef, seed=seed)
+    g.to_device(0)
+    want = g.count(4, warp_granularity=1)
+    assert [g.count(4, a) for a in ALGOS] == [want] * 3
+    roots = np.concatenate([np.arange(0, g.n, 3), [0, 1, 0]])  # some twice
+    assert g.count(4, roots=roots) == g.count(4, roots=roots, warp_granularity=3)
+
+
+# roots of the most neighbours the counters take and one more; several ranges
+# of counters; a root just under the least number of paths
+@pytest.mark.parametrize("d,n", [(1024, 1100), (1025, 1100), (700, 98304), (700, 98305), (900, 250000), (12, 200000)])
+def test_houses_of_a_hub_root(d, n):
+    rng = np.random.default_rng(d)
+    near = np.sort(rng.choice(np.arange(1, n), d, replace=False))
+    e = np.concatenate([np.stack([np.zeros(d, np.int64), near], 1), near[random_edges(d, 6 * d, 7)],
+                        np.stack([rng.choice(near, 20 * d), rng.integers(1, n, 20 * d)], 1)])
+    rp, cl = csr_of(n, e[e[:, 0] != e[:, 1]])
+    g = sme.Graph.from_csr(rp, cl)
+    g.to_device(0)
+    roots = [0, int(near[0]), int(near[-1]), int(near[d // 2]), 0]
+    want = g.count(4, roots=roots, warp_granularity=1)
+    assert want > 0
+    assert g.count(4, roots=roots) == want
