@@ -9,16 +9,17 @@
 // triangular (bit j of row i only for i < j), so a clique is counted once.
 // Nothing is materialised and nothing leaves the SM but the count.  Whole
 // calls, level program against this: 4-cliques of R-MAT s18 ef16, every root
-// 73.0 -> 2.2 ms; 5-cliques of the oriented R-MAT s17 ef16 187 -> 8.5 ms;
+// 73.0 -> 2.2 ms; 5-cliques of the oriented R-MAT s17 ef16 187 -> 5.6 ms;
 // 4-cliques of 16 384 roots of R-MAT s20 ef16 0.91 -> 0.40 ms.
 //
 // Few roots are bound by the latency of the build's loads (hub bitmap words
 // from HBM): hence four of them in flight per lane, 32 lists fetched at once
 // and many warps per root (4-cliques, s20 roots: 0.80 -> 0.40 ms).  Many roots
 // are bound by instruction issue: hence the candidates' hash table (1-2
-// shared-memory reads per looked-up element, a binary search takes 8) and the
+// shared-memory reads per looked-up element, a binary search takes 8), the
 // member lists compacted from their parent's by ballot (5-cliques, s17: 18 ->
-// 8.5 ms together; expanding the bits of every AND took the other half).
+// 8.5 ms together; expanding the bits of every AND took the other half) and,
+// on short rows, pairs of members instead of a warp per member (-> 5.6 ms).
 //
 // A root's cost grows with d, so roots are sorted into classes by d: up to 32
 // a warp and one word per row (k_clique_small); up to 256, 512 and 1024 (896
@@ -338,57 +339,111 @@ __device__ __forceinline__ uint32_t Expand(const uint32_t* row, uint32_t w0, uin
   return total;
 }
 
+// A row of the matrix is an odd number of units, so that rows spread over the
+// banks.  The unit is a word, except in class M for k >= 5, whose inner loop
+// is the pairs below: there it is a 16-byte quad, four words per load and loop
+// step (5-cliques of the oriented R-MAT s17: class M 4.0-4.3 ms with quads and
+// pairs, 6.0 without; 4-cliques and class L, whose rows are read from the
+// middle on, are faster on words: 1.5 against 1.7 and 1.2 against 1.5 ms).
+constexpr bool CliqueQuads(int k, int threads, bool global) {
+  return k >= 5 && threads == kCliqueMThreads && !global;
+}
+template <bool QUADS>
+struct RowUnit {
+  typedef uint32_t T;
+  static constexpr int kShift = 5;  // log2 of a unit's bits
+  static __device__ __forceinline__ uint32_t And(uint32_t x, uint32_t y) { return x & y; }
+  static __device__ __forceinline__ uint32_t Pop(uint32_t x) { return __popc(x); }
+  static __device__ __forceinline__ uint32_t Zero() { return 0; }
+};
+template <>
+struct RowUnit<true> {
+  typedef uint4 T;
+  static constexpr int kShift = 7;
+  static __device__ __forceinline__ uint4 And(const uint4& x, const uint4& y) {
+    return make_uint4(x.x & y.x, x.y & y.y, x.z & y.z, x.w & y.w);
+  }
+  static __device__ __forceinline__ uint32_t Pop(const uint4& x) {
+    return __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
+  }
+  static __device__ __forceinline__ uint4 Zero() { return make_uint4(0, 0, 0, 0); }
+};
+constexpr uint32_t RowUnits(uint32_t d, bool quads) { return quads ? (d + 127) / 128 : (d + 31) / 32; }
+
 // D-cliques inside the set S, whose nl members `list` holds, on the rows of
-// `mat`; lane-local partial counts.
-template <int D>
-__device__ __forceinline__ unsigned long long RowCliques(const uint32_t* S, const uint16_t* list, uint32_t nl,
-                                                         const uint32_t* mat, uint32_t ws, uint32_t W,
-                                                         uint16_t* lists, uint32_t lcap, uint32_t* sets,
-                                                         uint32_t wcap) {
+// `mat` (ws units apart, W units each); lane-local partial counts.
+template <int D, bool QUADS, typename T = typename RowUnit<QUADS>::T>
+__device__ __forceinline__ unsigned long long RowCliques(const T* S, const uint16_t* list, uint32_t nl,
+                                                         const T* mat, uint32_t ws, uint32_t W, uint16_t* lists,
+                                                         uint32_t lcap, T* sets, uint32_t wcap) {
+  typedef RowUnit<QUADS> U;
   const int lane = threadIdx.x & 31;
   unsigned long long c = 0;
   if constexpr (D == 2) {
     for (uint32_t t = lane; t < nl; t += 32) {
       const uint32_t l = list[t];
-      const uint32_t* row = mat + (size_t)l * ws;
+      const T* row = mat + (size_t)l * ws;
       uint32_t s = 0;
 #pragma unroll 4
-      for (uint32_t w = l >> 5; w < W; ++w) s += __popc(S[w] & row[w]);
+      for (uint32_t w = l >> U::kShift; w < W; ++w) s += U::Pop(U::And(S[w], row[w]));
       c += s;
     }
   } else {
+    if (QUADS && D == 3) {
+      // short rows: the pairs of members over the lanes, each joined pair
+      // counting the third members in S and both rows.  A warp per member
+      // leaves most lanes idle here (a member is joined to a dozen others).
+      const uint32_t pairs = nl * (nl - 1) / 2;
+      uint32_t t = 0, o = lane;  // pair (t, t + 1 + o)
+      for (uint32_t f = lane; f < pairs; f += 32, o += 32) {
+        while (o >= nl - 1 - t) {  // f < pairs: a row with pairs is left
+          o -= nl - 1 - t;
+          ++t;
+        }
+        const uint32_t l = list[t], x = list[t + 1 + o];
+        const T* row = mat + (size_t)l * ws;
+        if ((reinterpret_cast<const uint32_t*>(row)[x >> 5] >> (x & 31)) & 1u) {
+          const T* other = mat + (size_t)x * ws;
+          uint32_t s = 0;
+          for (uint32_t w = x >> U::kShift; w < W; ++w) s += U::Pop(U::And(U::And(S[w], row[w]), other[w]));
+          c += s;
+        }
+      }
+      return c;
+    }
     for (uint32_t t = 0; t + D - 1 < nl; ++t) {
       const uint32_t l = list[t];
-      const uint32_t* row = mat + (size_t)l * ws;
+      const T* row = mat + (size_t)l * ws;
       __syncwarp();  // the previous round's set and list are read out
-      for (uint32_t w = (l >> 5) + lane; w < W; w += 32) sets[w] = S[w] & row[w];
+      for (uint32_t w = (l >> U::kShift) + lane; w < W; w += 32) sets[w] = U::And(S[w], row[w]);
       // the members after l that l is joined to
       uint32_t n2 = 0;
       for (uint32_t k0 = t + 1; k0 < nl; k0 += 32) {
         const uint32_t k = k0 + lane;
         const uint32_t x = k < nl ? list[k] : 0;
-        const bool in = k < nl && ((row[x >> 5] >> (x & 31)) & 1u);
+        const bool in = k < nl && ((reinterpret_cast<const uint32_t*>(row)[x >> 5] >> (x & 31)) & 1u);
         const unsigned mask = __ballot_sync(FULL, in);
         if (in) lists[n2 + __popc(mask & ((1u << lane) - 1))] = (uint16_t)x;
         n2 += __popc(mask);
       }
       __syncwarp();
       if (n2 >= D - 1)
-        c += RowCliques<D - 1>(sets, lists, n2, mat, ws, W, lists + lcap, lcap, sets + wcap, wcap);
+        c += RowCliques<D - 1, QUADS>(sets, lists, n2, mat, ws, W, lists + lcap, lcap, sets + wcap, wcap);
     }
   }
   return c;
 }
 
-// Shared memory of a CTA: the matrix (unless it is in global scratch), the
-// candidates and their table (not with the matrix in scratch), and per warp
-// K - 3 member lists and K - 4 sets.
+// Shared memory of a CTA: the matrix (unless it is in global scratch), per warp
+// K - 4 sets, the candidates and their table (not with the matrix in scratch),
+// and per warp K - 3 member lists.
 constexpr size_t CliqueSmem(int k, uint32_t dmax, int threads, bool global) {
-  const size_t W = (dmax + 31) / 32, ws = W | 1, warps = threads / 32;
-  return (global ? 0 : (size_t)dmax * ws * 4) + (size_t)dmax * 4 + warps * (k - 4) * W * 4 + (global ? 0 : (size_t)6 << TableLg(dmax)) +
-         warps * (k - 3) * (size_t)dmax * 2 + 64;
+  const bool quads = CliqueQuads(k, threads, global);
+  const size_t W = RowUnits(dmax, quads), unit = quads ? 16 : 4, warps = threads / 32;
+  return (global ? 0 : (size_t)dmax * (W | 1) * unit) + warps * (k - 4) * W * unit + (size_t)dmax * 4 +
+         (global ? 0 : (size_t)6 << TableLg(dmax)) + warps * (k - 3) * (size_t)dmax * 2;
 }
-constexpr size_t CliqueScratchWords(uint32_t dmax) { return (size_t)dmax * (((dmax + 31) / 32) | 1); }
+constexpr size_t CliqueScratchWords(uint32_t dmax) { return (size_t)dmax * (RowUnits(dmax, false) | 1); }
 
 template <int K, bool ORIENT, int THREADS, bool GLOBAL>
 __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t* __restrict__ roots,
@@ -396,19 +451,22 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
                                                         const uint32_t* __restrict__ nq, uint32_t cap,
                                                         uint32_t* next, uint32_t dmax, uint32_t* scratch,
                                                         unsigned long long* acc) {
-  extern __shared__ uint32_t cq_sh[];
+  extern __shared__ uint4 cq_sh[];
   constexpr int WARPS = THREADS / 32;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const uint32_t wcap = (dmax + 31) / 32;
-  uint32_t* mat = GLOBAL ? scratch + (size_t)blockIdx.x * CliqueScratchWords(dmax) : cq_sh;
-  uint32_t* R = GLOBAL ? cq_sh : cq_sh + (size_t)dmax * (wcap | 1);
+  constexpr bool QUADS = CliqueQuads(K, THREADS, GLOBAL);
+  typedef typename RowUnit<QUADS>::T Unit;
+  constexpr uint32_t kWords = sizeof(Unit) / 4;
+  const uint32_t wcap = RowUnits(dmax, QUADS);
+  Unit* sh = reinterpret_cast<Unit*>(cq_sh);
+  Unit* mat = GLOBAL ? reinterpret_cast<Unit*>(scratch + (size_t)blockIdx.x * CliqueScratchWords(dmax)) : sh;
+  Unit* sets0 = GLOBAL ? sh : sh + (size_t)dmax * (wcap | 1);
+  Unit* sets = sets0 + (size_t)wid * (K - 4) * wcap;
+  uint32_t* R = reinterpret_cast<uint32_t*>(sets0 + (size_t)WARPS * (K - 4) * wcap);
   const uint32_t tlg = TableLg(dmax);
   uint32_t* keys = R + dmax;
   uint16_t* at = reinterpret_cast<uint16_t*>(keys + (1u << tlg));
-  uint32_t* sets0 = GLOBAL ? R + dmax : keys + (3u << (tlg - 1));
-  uint32_t* sets = sets0 + (size_t)wid * (K - 4) * wcap;
-  uint16_t* lists = reinterpret_cast<uint16_t*>(sets0 + (size_t)WARPS * (K - 4) * wcap) +
-                    (size_t)wid * (K - 3) * dmax;
+  uint16_t* lists = (GLOBAL ? reinterpret_cast<uint16_t*>(keys) : at + (1u << tlg)) + (size_t)wid * (K - 3) * dmax;
   __shared__ uint32_t s_item, s_row;
   const uint32_t count = min(*nq, cap);
   unsigned long long local = 0, bytes = 0;
@@ -432,9 +490,10 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
       d -= r0;
     }
     const uint32_t parts = CliqueParts(K, d);
-    const uint32_t W = (d + 31) / 32, ws = W | 1;  // odd stride: rows spread over the banks
+    const uint32_t W = RowUnits(d, QUADS), ws = W | 1;
+    uint32_t* bits_of = reinterpret_cast<uint32_t*>(mat);  // row i's words start at i * ws * kWords
     for (uint32_t i = tid; i < d; i += THREADS) R[i] = __ldg(L + i);
-    for (uint32_t i = tid; i < d * ws; i += THREADS) mat[i] = 0;
+    for (uint32_t i = tid; i < d * ws; i += THREADS) mat[i] = RowUnit<QUADS>::Zero();
     if (!GLOBAL) {
       for (uint32_t i = tid; i < (1u << tlg); i += THREADS) keys[i] = kNoKey;
       __syncthreads();
@@ -477,7 +536,7 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
               const unsigned bits = __ballot_sync(FULL, (word[t] >> (x[t] & 31)) & 1u);
-              if (lane == 0 && bits) mat[(size_t)i * ws + (jb >> 5) + t] = bits;  // only this warp writes row i here
+              if (lane == 0 && bits) bits_of[(size_t)i * ws * kWords + (jb >> 5) + t] = bits;  // row i is this warp's
             }
           }
           if (lane == 0) bytes += 12ULL + 8ULL * (d - i);
@@ -490,7 +549,7 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
               in = pos < len && __ldg(a + pos) == x;
             }
             const unsigned bits = __ballot_sync(FULL, in);
-            if (lane == 0 && bits) mat[(size_t)i * ws + (jb >> 5)] = bits;
+            if (lane == 0 && bits) bits_of[(size_t)i * ws * kWords + (jb >> 5)] = bits;
           }
           if (lane == 0) bytes += 12ULL + 8ULL * (d - i);
         } else {
@@ -510,7 +569,7 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
               }
               if (c < d && (ORIENT || c > i)) {
                 const uint32_t lo = min(i, c), hi = max(i, c);
-                atomicOr(mat + (size_t)lo * ws + (hi >> 5), 1u << (hi & 31));
+                atomicOr(bits_of + (size_t)lo * ws * kWords + (hi >> 5), 1u << (hi & 31));
               }
             }
           }
@@ -524,12 +583,12 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
       if (lane == 0) i = atomicAdd(&s_row, 1u);
       i = __shfl_sync(FULL, i, 0) * parts + part;
       if (i >= d) break;
-      const uint32_t* row = mat + (size_t)i * ws;
+      const Unit* row = mat + (size_t)i * ws;
       __syncwarp();
-      const uint32_t nl = Expand(row, i >> 5, W, lists);
+      const uint32_t nl = Expand(reinterpret_cast<const uint32_t*>(row), i >> 5, W * kWords, lists);
       __syncwarp();
       if (nl >= K - 2)
-        local += RowCliques<K - 2>(row, lists, nl, mat, ws, W, lists + dmax, dmax, sets, wcap);
+        local += RowCliques<K - 2, QUADS>(row, lists, nl, mat, ws, W, lists + dmax, dmax, sets, wcap);
     }
     __syncthreads();  // the matrix is rebuilt for the next root
   }

@@ -100,7 +100,7 @@ def test_cliques_of_complete_graphs(n, ks):
 
 # vertex 0 sees every other vertex: a root of d candidates in every class, and
 # above the last one, which keeps the level program
-@pytest.mark.parametrize("d", [31, 256, 257, 700, 896, 897, 1024, 1025, 4096, 4097, 5000])
+@pytest.mark.parametrize("d", [31, 256, 257, 700, 896, 897, 960, 961, 1024, 1025, 4096, 4097, 5000])
 @pytest.mark.parametrize("q", [3, 7, 11])
 def test_cliques_of_a_hub_root(d, q):
     e = np.concatenate([np.stack([np.zeros(d, np.int64), np.arange(1, d + 1)], 1), 1 + random_edges(d, 14 * d, d)])
