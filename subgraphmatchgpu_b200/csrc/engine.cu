@@ -99,12 +99,14 @@ __device__ uint64_t BlockExclusiveScan(uint64_t v, uint64_t* total) {
 //           src/gpu/impl/light/ext/EXTLIGHTOrganizeBatch.cuh:11-53)
 //   E_SET   the size of u's candidate set
 //   E_CHILD the children of the path when u is materialised: the set's range
-//           clipped by < and >, minus the excluded values in it
+//           clipped by < and >, minus the excluded values in it (`first`, when
+//           given, receives where the range starts)
 enum EstKind { E_LIST, E_SET, E_CHILD };
 
 template <EstKind KIND>
 __device__ __forceinline__ uint64_t EstOf(const DFront& F, const DStep& s, const DCond& c,
-                                          const uintE* __restrict__ rp, uint32_t p, uint64_t* lists) {
+                                          const uintE* __restrict__ rp, uint32_t p, uint64_t* lists,
+                                          uint32_t* first) {
   if (KIND == E_LIST) {
     uint64_t m = ~0ULL, sd = 0;
     for (int i = 0; i < s.nconn; ++i) {
@@ -129,6 +131,7 @@ __device__ __forceinline__ uint64_t EstOf(const DFront& F, const DStep& s, const
   Bounds bd = MakeBounds(c, F, p);
   uint32_t r0, r1, ex[MAXV];
   Range(a, n, bd, r0, r1);
+  if (first) first[p] = r0;
   return (uint64_t)(r1 - r0 - Exclusions(a, r0, r1, bd, ex));
 }
 
@@ -143,7 +146,8 @@ constexpr uint32_t kScanSmall = 148 * 4 * SCAN_THREADS;
 template <EstKind KIND, bool TWO, int ITEMS>
 __global__ void __launch_bounds__(SCAN_THREADS) k_est_scan(DFront F, DStep s, DCond c,
                                                            const uintE* __restrict__ rp, uint64_t* out,
-                                                           uint64_t* out2, uint64_t* bs, uint32_t* ticket) {
+                                                           uint64_t* out2, uint32_t* first, uint64_t* bs,
+                                                           uint32_t* ticket) {
   const uint64_t base = (uint64_t)blockIdx.x * (SCAN_THREADS * ITEMS);
   const uint32_t nb = gridDim.x;
   uint64_t v[ITEMS], v2[TWO ? ITEMS : 1];
@@ -151,7 +155,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_est_scan(DFront F, DStep s, DC
   for (int k = 0; k < ITEMS; ++k) {
     const uint64_t i = base + (uint64_t)k * SCAN_THREADS + threadIdx.x;
     uint64_t lists = 0;
-    v[k] = i < F.P ? EstOf<KIND>(F, s, c, rp, (uint32_t)i, &lists) : 0;
+    v[k] = i < F.P ? EstOf<KIND>(F, s, c, rp, (uint32_t)i, &lists, first) : 0;
     if (TWO) v2[k] = lists;
   }
   uint64_t run = 0, run2 = 0;
@@ -1347,6 +1351,47 @@ __global__ void __launch_bounds__(WARP_BLOCK) k_mat_write_big(DFront F, DCond c,
   }
 }
 
+// The same without `!=` conditions, where a parent's children are one range of
+// its set starting at first[p] (null: at the set's start): one lane per child
+// row.  A warp takes `rows` consecutive rows, finds the parents of the first
+// and the last one together and each lane its row's between them, so neither
+// a long parent nor many short ones hold a warp up (a warp per parent waited
+// for its longest one, a warp per 1024 rows for its parents' set-up).  32 rows
+// while the warps fit the device, kMatRows beyond.  Triangles of R-MAT s14,
+// 114 000 rows: 73 us by the two kernels below and above, 10 us here.
+constexpr uint32_t kMatRows = 128;
+
+__global__ void __launch_bounds__(WARP_BLOCK) k_mat_rows(DFront F, DMatOut o, const uint64_t* __restrict__ incl,
+                                                         const uint32_t* __restrict__ first, uint64_t total,
+                                                         uint32_t rows) {
+  const int lane = threadIdx.x & 31;
+  const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const int u = o.u;
+  for (uint64_t c0 = gw * rows; c0 < total; c0 += nw * rows) {
+    const uint64_t c1 = c0 + rows < total ? c0 + rows : total;
+    const uint32_t pa = WarpUpperBound64(incl, F.P, c0);
+    const uint32_t pb = pa + WarpUpperBound64(incl + pa, F.P - pa, c1 - 1);
+    for (uint64_t w = c0 + lane; w < c1; w += 32) {
+      uint32_t lo = pa, hi = pb;  // first p with incl[p] > w
+      while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        if (__ldg(incl + mid) > w) hi = mid;
+        else lo = mid + 1;
+      }
+      const uint64_t off = lo == 0 ? 0 : __ldg(incl + lo - 1);
+      const uint32_t s = SetIndex(F, u, lo);
+      const uint32_t* a = reinterpret_cast<const uint32_t*>(F.set[u].ptr[s]);
+      const uint32_t x = __ldg(a + (first ? __ldg(first + lo) : 0) + (uint32_t)(w - off));
+#pragma unroll
+      for (int i = 0; i < MAXV; ++i) {
+        if (i < o.nmat) o.inst[o.mat[i]][w] = o.mat[i] == u ? x : F.inst[o.mat[i]][lo];
+        if (i < o.nsets) o.cidx[o.sets[i]][w] = SetIndex(F, o.sets[i], lo);
+      }
+    }
+  }
+}
+
 // Parents of at most `big` children: one warp each (the large ones are
 // k_mat_write_big's).
 __global__ void __launch_bounds__(WARP_BLOCK) k_mat_write(DFront F, DCond c, DMatOut o,
@@ -1594,17 +1639,20 @@ __global__ void __launch_bounds__(WARP_BLOCK) k_ext_load(DFront F, DStep s, cons
   }
 }
 
-// Writes complete instances (all vertices materialised), in output slots.
-__global__ void k_emit(DFront F, uint8_t n, const uint8_t* __restrict__ slot_dummy, uint8_t s0,
-                       uint8_t s1, uint8_t s2, uint8_t s3, uint8_t s4, uint8_t s5, uint32_t* out,
-                       uint64_t cap, unsigned long long* counter) {
-  const uint8_t slot[MAXV] = {s0, s1, s2, s3, s4, s5};
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < F.P; p += gridDim.x * blockDim.x) {
-    unsigned long long pos = atomicAdd(counter, 1ULL);
-    if (pos < cap)
-      for (int v = 0; v < n; ++v) out[pos * n + slot[v]] = F.inst[v][p];
+// Writes complete instances (all vertices materialised) from instance `at` on,
+// in output slots: one thread per output word, so the writes are whole lines
+// (cols.p[s]: the column of output slot s).  The position of a frontier's
+// instances is the number emitted before it, which the host knows: no counter.
+struct EmitCols {
+  const uint32_t* p[MAXV];
+};
+__global__ void k_emit(EmitCols cols, uint32_t P, uint32_t n, uint64_t at, uint32_t* out, uint64_t cap) {
+  const uint64_t fit = at < cap ? (cap - at < P ? cap - at : P) : 0;
+  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < fit * n;
+       e += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t p = e / n;
+    out[at * n + e] = __ldg(cols.p[e - p * n] + p);
   }
-  (void)slot_dummy;
 }
 
 }  // namespace
@@ -1663,6 +1711,7 @@ void DestroyContext(DeviceContext* c) {
   if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
   if (c->arena.base) cudaFree(c->arena.base);
   if (c->h_pinned) cudaFreeHost(c->h_pinned);
+  if (c->h_stage) cudaFreeHost(c->h_stage);
   if (c->stream) cudaStreamDestroy(c->stream);
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
   for (auto e : c->copy_ev)
@@ -2265,8 +2314,8 @@ class Executor {
                              (h[3] & ENGINE_ERR_TIMEOUT ? " bulk-copy wait gave up" : "") + " (engine error flags " +
                              std::to_string(h[3]) + ")");
     RunResult r;
-    r.count = prog_.enumerate ? h[2] : h[0] - (h[8] - minus_paths_);
-    r.emitted = h[2];
+    r.count = prog_.enumerate ? emitted_ : h[0] - (h[8] - minus_paths_);
+    r.emitted = emitted_;
     r.stats.algorithmic_bytes = h[1] + h[9];
     r.stats.reuse_hits = h[5];
     ext_bytes_ += h[6] * 4;
@@ -2305,12 +2354,13 @@ class Executor {
   const std::vector<Step>* steps_;  // the level program being run
   int sms_ = 148;
   bool lists_simple_ = false;  // known to hold no element twice
-  // [0] count [1] bytes [2] emitted [3] error flags [4] list cache overflow
+  // [0] count [1] bytes [3] error flags [4] list cache overflow
   // [5] reuse hits [6] list cache elements [7] ticket of k_est_scan; [8..13]
   // count, bytes and hits of Program::minus
   static constexpr int kCtrl = 16;
   unsigned long long* ctrl_ = nullptr;
   unsigned long long* acc_ = nullptr;  // counters of the program being run
+  uint64_t emitted_ = 0;               // instances written (or counted past the capacity)
   uint64_t minus_paths_ = 0;           // paths of the last step of Program::minus
   uint64_t launches_ = 0, batches_ = 0, paths_ = 0, hot_ = 0, root_h2d_ = 0;
   const uint32_t* ext_cols_ = nullptr;
@@ -3005,13 +3055,15 @@ class Executor {
     uint64_t est, lists;
   };
   template <EstKind KIND, int ITEMS>
-  void LaunchEstScan(const DFront& F, const DStep& ds, const DCond& dc, uint64_t* est, uint64_t* est2, uint32_t nb,
-                     uint64_t* bs) {
+  void LaunchEstScan(const DFront& F, const DStep& ds, const DCond& dc, uint64_t* est, uint64_t* est2,
+                     uint32_t* first, uint32_t nb, uint64_t* bs) {
     uint32_t* ticket = (uint32_t*)(ctrl_ + 7);
     if (est2)
-      k_est_scan<E_LIST, true, ITEMS><<<nb, SCAN_THREADS, 0, st_>>>(F, ds, dc, g_.row_ptrs, est, est2, bs, ticket);
+      k_est_scan<E_LIST, true, ITEMS><<<nb, SCAN_THREADS, 0, st_>>>(F, ds, dc, g_.row_ptrs, est, est2, nullptr, bs,
+                                                                    ticket);
     else
-      k_est_scan<KIND, false, ITEMS><<<nb, SCAN_THREADS, 0, st_>>>(F, ds, dc, g_.row_ptrs, est, nullptr, bs, ticket);
+      k_est_scan<KIND, false, ITEMS><<<nb, SCAN_THREADS, 0, st_>>>(F, ds, dc, g_.row_ptrs, est, nullptr, first, bs,
+                                                                  ticket);
     Launched();
     if (nb == 1) return;
     if (est2) k_scan_add<true, ITEMS><<<nb - 1, SCAN_THREADS, 0, st_>>>(est, est2, F.P, bs);
@@ -3019,13 +3071,14 @@ class Executor {
     Launched();
   }
   template <EstKind KIND>
-  Totals EstScan(const DFront& F, const DStep& ds, const DCond& dc, uint64_t* est, uint64_t* est2) {
+  Totals EstScan(const DFront& F, const DStep& ds, const DCond& dc, uint64_t* est, uint64_t* est2,
+                 uint32_t* first = nullptr) {
     const uint32_t tile = F.P <= kScanSmall ? SCAN_THREADS : SCAN_TILE;
     const uint32_t nb = (F.P + tile - 1) / tile;
     const size_t m = A_.Mark();
     uint64_t* bs = (uint64_t*)A_.Alloc(((size_t)nb + 1) * 16);
-    if (tile == SCAN_THREADS) LaunchEstScan<KIND, 1>(F, ds, dc, est, est2, nb, bs);
-    else LaunchEstScan<KIND, SCAN_ITEMS>(F, ds, dc, est, est2, nb, bs);
+    if (tile == SCAN_THREADS) LaunchEstScan<KIND, 1>(F, ds, dc, est, est2, first, nb, bs);
+    else LaunchEstScan<KIND, SCAN_ITEMS>(F, ds, dc, est, est2, first, nb, bs);
     CK(cudaMemcpyAsync(ctx_.h_pinned, bs + nb, 8, cudaMemcpyDeviceToHost, st_));
     if (est2) CK(cudaMemcpyAsync(ctx_.h_pinned + 1, bs + 2 * nb + 1, 8, cudaMemcpyDeviceToHost, st_));
     CK(cudaStreamSynchronize(st_));
@@ -3084,11 +3137,13 @@ class Executor {
   }
 
   void Emit(const DFront& F) {
-    uint8_t sl[MAXV] = {0, 0, 0, 0, 0, 0};
-    for (int v = 0; v < prog_.n; ++v) sl[v] = prog_.out_slot[v];
-    k_emit<<<Grid(F.P, 256), 256, 0, st_>>>(F, (uint8_t)prog_.n, nullptr, sl[0], sl[1], sl[2], sl[3],
-                                            sl[4], sl[5], out_, cap_, ctrl_ + 2);
-    Launched();
+    EmitCols cols{};
+    for (int v = 0; v < prog_.n; ++v) cols.p[prog_.out_slot[v]] = F.inst[v];
+    if (emitted_ < cap_) {
+      k_emit<<<Grid((uint64_t)F.P * prog_.n, 256), 256, 0, st_>>>(cols, F.P, (uint32_t)prog_.n, emitted_, out_, cap_);
+      Launched();
+    }
+    emitted_ += F.P;
   }
 
   void ClipViews(const DFront& F, const DStep& ds, const DGraph& G, uint64_t* ptr, uint32_t* cnt) {
@@ -3098,9 +3153,21 @@ class Executor {
     Launched();
   }
 
+  static bool HasNe(const DCond& c) {
+    for (int i = 0; i < c.n; ++i)
+      if (c.op[i] == 2) return true;
+    return false;
+  }
+  // Where each path's children start in its set: needed when conditions clip
+  // the set and none excludes single values.
+  uint32_t* FirstOf(const DCond& dc, uint32_t P) {
+    return dc.n && !HasNe(dc) ? (uint32_t*)A_.Alloc((size_t)P * 4) : nullptr;
+  }
+
   // Expands the paths of F into their C children (`cnt`: inclusive child
-  // counts) and runs the next level on them.
-  void Materialize(size_t k, const DFront& F, const DCond& dc, const uint64_t* cnt, uint64_t C) {
+  // counts, `first`: see FirstOf) and runs the next level on them.
+  void Materialize(size_t k, const DFront& F, const DCond& dc, const uint64_t* cnt, const uint32_t* first,
+                   uint64_t C) {
     if (C == 0) return;
     if (C > 0x7fffffffULL) Fail(SME_ERR_OOM, "materialised batch exceeds 2^31 partial instances");
     const Step& s = (*steps_)[k];
@@ -3119,12 +3186,18 @@ class Executor {
       o.cidx[s.sets_after[i]] = (uint32_t*)A_.Alloc(C * 4);
     }
     Timed tm = TimerStart();
-    k_mat_write<<<WarpGrid(F.P), WARP_BLOCK, 0, st_>>>(F, dc, o, cnt, C, kMatBig, err);
-    Launched();
-    if (C > kMatBig) {  // else no parent has more
-      k_mat_write_big<<<WarpGrid((C + kMatChunk - 1) / kMatChunk), WARP_BLOCK, 0, st_>>>(F, dc, o, cnt, C, kMatBig,
-                                                                                         err);
+    if (!HasNe(dc)) {
+      const uint32_t rows = C <= (uint64_t)sms_ * 64 * 32 ? 32 : kMatRows;
+      k_mat_rows<<<WarpGrid((C + rows - 1) / rows), WARP_BLOCK, 0, st_>>>(F, o, cnt, first, C, rows);
       Launched();
+    } else {
+      k_mat_write<<<WarpGrid(F.P), WARP_BLOCK, 0, st_>>>(F, dc, o, cnt, C, kMatBig, err);
+      Launched();
+      if (C > kMatBig) {  // else no parent has more
+        k_mat_write_big<<<WarpGrid((C + kMatChunk - 1) / kMatChunk), WARP_BLOCK, 0, st_>>>(F, dc, o, cnt, C, kMatBig,
+                                                                                           err);
+        Launched();
+      }
     }
     TimerStop(tm, kPhaseMaterialize);
     DFront Fn{};
@@ -3214,8 +3287,7 @@ class Executor {
     }
     const size_t mark0 = A_.Mark();
     const DCond dc = ToDCond(s.cond);
-    bool has_ne = false;
-    for (int i = 0; i < dc.n; ++i) has_ne |= dc.op[i] == 2;
+    const bool has_ne = HasNe(dc);
     uint64_t* est = nullptr;
     uint64_t* sumdeg = nullptr;  // external mode: list elements per path
     std::vector<Batch> batches;
@@ -3231,12 +3303,13 @@ class Executor {
       // set sizes, an upper bound, each counted in its turn
       Timed to = TimerStart();
       uint64_t* cnt = (uint64_t*)A_.Alloc((size_t)F.P * 8);
-      const Totals t = EstScan<E_CHILD>(F, ds, dc, cnt, nullptr);
+      uint32_t* first = FirstOf(dc, F.P);
+      const Totals t = EstScan<E_CHILD>(F, ds, dc, cnt, nullptr, first);
       TimerStop(to, kPhaseOrganize);
       const double pf = 16, cf = 4.0 * (s.mat_after.size() + s.sets_after.size()) + 16;
       if (pf * F.P + cf * (double)t.est <= (double)Budget(k) && t.est <= 2000000000ull) {
         ++batches_;
-        Materialize(k, F, dc, cnt, t.est);
+        Materialize(k, F, dc, cnt, first, t.est);
         A_.Release(mark0);
         return;
       }
@@ -3315,9 +3388,10 @@ class Executor {
         case S_MATERIALIZE: {
           uint64_t* cnt = (uint64_t*)A_.Alloc((size_t)Pb * 8);
           Timed tm = TimerStart();
-          const uint64_t C = EstScan<E_CHILD>(Fb, ds, dc, cnt, nullptr).est;
+          uint32_t* first = FirstOf(dc, Pb);
+          const uint64_t C = EstScan<E_CHILD>(Fb, ds, dc, cnt, nullptr, first).est;
           TimerStop(tm, kPhaseMaterialize);
-          Materialize(k, Fb, dc, cnt, C);
+          Materialize(k, Fb, dc, cnt, first, C);
           break;
         }
         default:

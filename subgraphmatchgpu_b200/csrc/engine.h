@@ -43,6 +43,8 @@ struct Arena {
 // Byte ranges a per-call packed upload is cut into (copy and expansion overlap).
 constexpr int kUploadChunks = 8;
 
+constexpr size_t kStageBytes = 4 << 20;
+
 // Per-device execution context: stream, arena, pinned staging buffers.
 struct DeviceContext {
   int device = 0;
@@ -53,6 +55,9 @@ struct DeviceContext {
   Arena arena;
   uint64_t* h_pinned = nullptr;  // small pinned host buffer for batch bounds
   size_t pinned_words = 0;
+  // pinned staging of enumerated instances, two halves of kStageBytes, made by
+  // the first enumeration that is long enough to use it
+  uint8_t* h_stage = nullptr;
   ~DeviceContext();
 };
 
