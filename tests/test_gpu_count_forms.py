@@ -200,3 +200,27 @@ def test_houses_of_a_hub_root(d, n):
     want = g.count(4, roots=roots, warp_granularity=1)
     assert want > 0
     assert g.count(4, roots=roots) == want
+
+
+@pytest.mark.parametrize("cap", [0, 1, 1000, 90000, 300000])
+def test_enumeration_copies_up_to_the_capacity(cap):
+    # 161 700 triangles (1.9 MB: the staged copy), and below its threshold
+    g = sme.Graph.clique(100)
+    out = np.full((max(cap, 1), 3), 0xFFFFFFFF, np.uint32)
+    import ctypes as C
+    n = C.c_uint64()
+    o = sme.opts(0)
+    st = sme.lib().sme_enumerate(g.handle, C.byref(o), out.ctypes.data, cap, C.byref(n))
+    assert n.value == comb(100, 3)
+    assert st == (0 if cap >= n.value else 8)
+    got = out[:min(cap, n.value)]
+    assert len(np.unique(got.astype(np.int64) @ [10000, 100, 1])) == len(got)
+    assert (got < 100).all() and (got[:, 0] < got[:, 1]).all() and (got[:, 1] < got[:, 2]).all()
+    assert (out[min(cap, n.value):] == 0xFFFFFFFF).all()
+
+
+def test_enumeration_over_several_staging_halves():
+    g = sme.Graph.clique(60)  # 487 635 4-cliques, 7.8 MB
+    inst = g.enumerate(3)
+    key = np.sort(inst.astype(np.int64) @ [216000, 3600, 60, 1])
+    assert len(np.unique(key)) == comb(60, 4) == len(inst)
