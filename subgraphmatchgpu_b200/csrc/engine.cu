@@ -2369,6 +2369,7 @@ class Executor {
   uint32_t* ext_cache_ = nullptr;    // device list cache
   uint64_t ext_cap_ = 0, ext_bound_ = 0;
   double ext_overlap_ = 32.0;
+  int ext_misses_ = 0;  // counting frontiers whose lists did not fit at once
 
   // The resident graph with its hub bitmaps (`use_bitmaps_` false: lists only).
   DGraph Resident() const {
@@ -3233,7 +3234,17 @@ class Executor {
           A_.Release(mg);
           return;
         }
-        // external: batches whose required lists fit the level budget
+        // external: the whole frontier when its lists fit the cache (they are
+        // shared by most of its paths, so this is tried before anything is
+        // estimated, while it keeps working), else batches whose lists do
+        if (ext_misses_ < 4) {
+          if (LoadLists(F, ds, ~0ull >> 1)) {
+            ++batches_;
+            Compute<1>(F, ds, View(), nullptr, 0, nullptr, nullptr, nullptr, 0);
+            return;
+          }
+          ++ext_misses_;
+        }
         const size_t m0 = A_.Mark();
         uint64_t* est = (uint64_t*)A_.Alloc((size_t)F.P * 8);
         uint64_t* sd = (uint64_t*)A_.Alloc((size_t)F.P * 8);
