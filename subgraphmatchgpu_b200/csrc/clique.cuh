@@ -1,13 +1,15 @@
-// k-cliques (k = 4, 5, 6) of a root task on bit matrices (device code).
+// k-cliques (k = 3 to 6) of a root task on bit matrices (device code).
 //
-// The level programs of Q3, Q7 and Q11 hold every triangle (and, for the
+// The level programs of Q0, Q3, Q7 and Q11 hold every edge, triangle (and, for the
 // larger cliques, every 4- and 5-clique) as a path and intersect lists once
 // per path.  Here a root's candidates R = N(u0) above u0 (d of them) get a
 // d x d bit matrix of the edges among them, built by one intersection per
 // candidate; the (k-1)-cliques of R are then counted on its rows: k - 3 levels
 // of one AND of two rows each and a last one of AND + popcount.  Rows are
 // triangular (bit j of row i only for i < j), so a clique is counted once.
-// Nothing is materialised and nothing leaves the SM but the count.  Whole
+// Triangles need no matrix, the build's hits are the count; they come here
+// only as a task of every root (see ORIENT).  Nothing is
+// materialised and nothing leaves the SM but the count.  Whole
 // calls, level program against this: 4-cliques of R-MAT s18 ef16, every root
 // 73.0 -> 2.2 ms; 5-cliques of the oriented R-MAT s17 ef16 187 -> 5.6 ms;
 // 4-cliques of 16 384 roots of R-MAT s20 ef16 0.91 -> 0.40 ms.
@@ -60,40 +62,50 @@ __device__ __forceinline__ void CList(const CView& V, uint32_t v, const uint32_t
 
 // ---- orientation by (degree, id) ------------------------------------------------
 constexpr int ORI_THREADS = 256;
-constexpr uint32_t kOriWarp = 512;                               // edges a warp takes
-constexpr uint32_t kOriTile = kOriWarp * (ORI_THREADS / 32);     // edges a CTA takes
+// Edges a warp takes: a chain of loads per 32 of them, so few while the graph
+// is small (R-MAT s14, 230 000 edges: 27 + 42 us with 512, 8 + 11 with 64).
+__host__ __device__ constexpr uint32_t OriWarp(uint64_t m) { return m < (4u << 20) ? 64 : 512; }
+constexpr uint32_t OriTile(uint64_t m) { return OriWarp(m) * (ORI_THREADS / 32); }  // edges a CTA takes
 
 __device__ __forceinline__ bool KeepsEdge(const uint64_t* rp, uint32_t u, uint64_t du, uint32_t x) {
   const uint64_t dx = __ldg(rp + x + 1) - __ldg(rp + x);
   return dx > du || (dx == du && x > u);
 }
 
-// FILL 0: kept edges per tile into bs; FILL 1: bs holds their exclusive sums,
-// the kept edges are written to ocols and every list's range to rng (cleared
-// by the caller, so an empty list's range is empty).
+// FILL 0: one bit per edge into `keep` and the kept edges per tile into bs;
+// FILL 1: bs holds their exclusive sums, the kept edges are written to ocols
+// and every list's range to rng (cleared by the caller, so an empty list's
+// range is empty).  Only the first pass gathers degrees.
 template <bool FILL>
 __global__ void __launch_bounds__(ORI_THREADS) k_orient(const uint64_t* __restrict__ rp,
                                                         const uint32_t* __restrict__ cols, uint32_t n, uint64_t m,
-                                                        uint64_t* bs, uint32_t* ocols, uint2* rng) {
+                                                        uint32_t* keep, uint64_t* bs, uint32_t* ocols, uint2* rng) {
   __shared__ uint32_t wkept[ORI_THREADS / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const uint64_t c0 = (uint64_t)blockIdx.x * kOriTile + (uint64_t)wid * kOriWarp;
-  const uint64_t c1 = c0 + kOriWarp < m ? c0 + kOriWarp : m;
-  uint32_t kept = 0, flags = 0, u0 = 0;
-  if (c0 < m) {
-    u0 = WarpOwner(rp, n, c0);
-    uint32_t u = u0;
-    for (uint32_t k = 0; k < kOriWarp / 32; ++k) {
-      const uint64_t e = c0 + k * 32 + lane;
-      bool keep = false;
-      if (e < c1) {
-        while (__ldg(rp + u + 1) <= e) ++u;  // ends: rp[n] = m > e
-        keep = KeepsEdge(rp, u, __ldg(rp + u + 1) - __ldg(rp + u), __ldg(cols + e));
+  const uint32_t per = OriWarp(m);
+  const uint64_t c0 = ((uint64_t)blockIdx.x * (ORI_THREADS / 32) + wid) * per;
+  const uint64_t c1 = c0 + per < m ? c0 + per : m;
+  uint32_t kept = 0, mine = 0;  // mine: the warp's bits, lane k those of its k-th 32 edges
+  if (FILL && c0 + 32ull * lane < c1 && lane < per / 32) mine = __ldg(keep + (c0 >> 5) + lane);
+  uint32_t u = c0 < m ? WarpOwner(rp, n, c0) : 0;
+  if (!FILL) {
+    if (c0 < m) {
+#pragma unroll 4
+      for (uint32_t k = 0; k < per / 32; ++k) {
+        const uint64_t e = c0 + k * 32 + lane;
+        bool yes = false;
+        if (e < c1) {
+          const uint32_t x = __ldg(cols + e);
+          while (__ldg(rp + u + 1) <= e) ++u;  // ends: rp[n] = m > e
+          yes = KeepsEdge(rp, u, __ldg(rp + u + 1) - __ldg(rp + u), x);
+        }
+        const uint32_t bits = __ballot_sync(FULL, yes);
+        if (lane == k) mine = bits;
       }
-      kept += __popc(__ballot_sync(FULL, keep));
-      flags |= (keep ? 1u : 0u) << k;
+      if (lane < per / 32 && c0 + 32ull * lane < c1) keep[(c0 >> 5) + lane] = mine;
     }
   }
+  kept = __reduce_add_sync(FULL, (unsigned)__popc(mine));
   if (lane == 0) wkept[wid] = kept;
   __syncthreads();
   if (!FILL) {
@@ -107,19 +119,18 @@ __global__ void __launch_bounds__(ORI_THREADS) k_orient(const uint64_t* __restri
   uint64_t at = bs[blockIdx.x];
   for (int w = 0; w < wid; ++w) at += wkept[w];
   if (c0 >= m) return;
-  uint32_t u = u0;
-  for (uint32_t k = 0; k < kOriWarp / 32; ++k) {
+  for (uint32_t k = 0; k < per / 32; ++k) {
     const uint64_t e = c0 + k * 32 + lane;
-    const bool keep = (flags >> k) & 1;
-    const unsigned mask = __ballot_sync(FULL, keep);
-    const uint32_t pos = (uint32_t)at + __popc(mask & ((1u << lane) - 1));
+    const uint32_t bits = __shfl_sync(FULL, mine, k);
+    const bool yes = (bits >> lane) & 1;
+    const uint32_t pos = (uint32_t)at + __popc(bits & ((1u << lane) - 1));
     if (e < c1) {
       while (__ldg(rp + u + 1) <= e) ++u;
-      if (keep) ocols[pos] = __ldg(cols + e);
+      if (yes) ocols[pos] = __ldg(cols + e);
       if (e == __ldg(rp + u)) rng[u].x = pos;
-      if (e + 1 == __ldg(rp + u + 1)) rng[u].y = pos + (keep ? 1 : 0);
+      if (e + 1 == __ldg(rp + u + 1)) rng[u].y = pos + (yes ? 1 : 0);
     }
-    at += __popc(mask);
+    at += __popc(bits);
   }
 }
 
@@ -134,6 +145,7 @@ constexpr uint32_t kPartShift = 29;  // queue entries: root index | part << 29
 // than the matrix each part builds.
 __device__ __forceinline__ uint32_t CliqueParts(int k, uint32_t d) {
   if (d <= kCliqueM) return 1;
+  if (k == 3) return min((uint32_t)kCliqueParts, (d + 127) / 128);
   if (k == 4) return d <= 1024 ? 1 : min(8u, (d + 511) / 512);
   return min((uint32_t)kCliqueParts, (d + 127) / 128);
 }
@@ -195,6 +207,23 @@ __global__ void __launch_bounds__(256) k_clique_classify(CView V, const uint32_t
   }
 }
 
+// Two lower bounds at once (LowerBound's steps, the loads of both in flight).
+__device__ __forceinline__ void LowerBound2(const uint32_t* a, uint32_t na, uint32_t x, const uint32_t* b, uint32_t nb,
+                                            uint32_t y, uint32_t& ra, uint32_t& rb) {
+  const uint32_t *pa = a, *pb = b;
+  uint32_t ca = na, cb = nb;
+  while (ca > 1 || cb > 1) {
+    const uint32_t ha = ca >> 1, hb = cb >> 1;  // 0 once one is down to an element
+    const uint32_t va = ha ? __ldg(pa + ha) : 0xFFFFFFFFu, vb = hb ? __ldg(pb + hb) : 0xFFFFFFFFu;
+    pa = va < x ? pa + ha : pa;
+    pb = vb < y ? pb + hb : pb;
+    ca -= ha;
+    cb -= hb;
+  }
+  ra = na ? (uint32_t)(pa - a) + (__ldg(pa) < x ? 1u : 0u) : 0;
+  rb = nb ? (uint32_t)(pb - b) + (__ldg(pb) < y ? 1u : 0u) : 0;
+}
+
 // ---- up to 32 candidates: a warp each ----------------------------------------------
 template <int K>
 __device__ __forceinline__ unsigned long long SmallCliques(const uint32_t* rows, uint32_t s) {
@@ -245,34 +274,48 @@ __global__ void __launch_bounds__(WARP_BLOCK, 6) k_clique_small(CView V, const u
     rows[lane] = 0;
     __syncwarp();
     const uint32_t np = d * (d - 1) / 2;
-    for (uint32_t f0 = 0; f0 < np; f0 += 32) {
-      const uint32_t f = f0 + lane;
-      uint32_t b = (uint32_t)((1.0f + sqrtf(1.0f + 8.0f * (float)f)) * 0.5f);
-      while (b * (b - 1) / 2 > f) --b;
-      while ((b + 1) * b / 2 <= f) ++b;
-      const uint32_t a = f - b * (b - 1) / 2;  // pair a < b
-      const uint32_t xa = __shfl_sync(FULL, x, a & 31), xb = __shfl_sync(FULL, x, b & 31);
-      uint32_t src = a & 31, y = xb;
-      if (ORIENT) {
-        const uint32_t da = __shfl_sync(FULL, deg, a & 31), db = __shfl_sync(FULL, deg, b & 31);
-        if (db < da || (db == da && xb < xa)) {
-          src = b & 31;
-          y = xa;
+    for (uint32_t f0 = 0; f0 < np; f0 += 64) {
+      // two pairs per lane, their searches side by side
+      uint32_t lo[2], hi[2], want[2], sn[2];
+      const uint32_t* sp[2];
+      bool in[2];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const uint32_t f = f0 + t * 32 + lane;
+        uint32_t b = (uint32_t)((1.0f + sqrtf(1.0f + 8.0f * (float)f)) * 0.5f);
+        while (b * (b - 1) / 2 > f) --b;
+        while ((b + 1) * b / 2 <= f) ++b;
+        const uint32_t a = f - b * (b - 1) / 2;  // pair a < b
+        const uint32_t xa = __shfl_sync(FULL, x, a & 31), xb = __shfl_sync(FULL, x, b & 31);
+        uint32_t src = a & 31;
+        want[t] = xb;
+        if (ORIENT) {
+          const uint32_t da = __shfl_sync(FULL, deg, a & 31), db = __shfl_sync(FULL, deg, b & 31);
+          if (db < da || (db == da && xb < xa)) {
+            src = b & 31;
+            want[t] = xa;
+          }
+        }
+        sp[t] = reinterpret_cast<const uint32_t*>(__shfl_sync(FULL, (unsigned long long)(uintptr_t)lp, src));
+        sn[t] = __shfl_sync(FULL, ln, src);
+        const uint32_t* sb =
+            ORIENT ? nullptr
+                   : reinterpret_cast<const uint32_t*>(__shfl_sync(FULL, (unsigned long long)(uintptr_t)bm, src));
+        lo[t] = a;
+        hi[t] = b;
+        in[t] = false;
+        if (f >= np) sn[t] = 0;
+        if (sb && f < np) {  // a hub: its bitmap answers, nothing to search
+          in[t] = BitTest(sb, want[t]);
+          sn[t] = 0;
         }
       }
-      const uint64_t sp = __shfl_sync(FULL, (unsigned long long)(uintptr_t)lp, src);
-      const uint32_t sn = __shfl_sync(FULL, ln, src);
-      const uint64_t sb = ORIENT ? 0 : __shfl_sync(FULL, (unsigned long long)(uintptr_t)bm, src);
-      if (f < np) {
-        bool in;
-        if (sb) {
-          in = BitTest(reinterpret_cast<const uint32_t*>(sb), y);
-        } else {
-          const uint32_t* s = reinterpret_cast<const uint32_t*>(sp);
-          const uint32_t pos = LowerBound(s, sn, y);
-          in = pos < sn && __ldg(s + pos) == y;
-        }
-        if (in) atomicOr(rows + a, 1u << b);
+      uint32_t pos[2];
+      LowerBound2(sp[0], sn[0], want[0], sp[1], sn[1], want[1], pos[0], pos[1]);
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        if (pos[t] < sn[t] && __ldg(sp[t] + pos[t]) == want[t]) in[t] = true;
+        if (in[t]) atomicOr(rows + lo[t], 1u << hi[t]);
       }
     }
     __syncwarp();
@@ -440,7 +483,8 @@ __device__ __forceinline__ unsigned long long RowCliques(const T* S, const uint1
 constexpr size_t CliqueSmem(int k, uint32_t dmax, int threads, bool global) {
   const bool quads = CliqueQuads(k, threads, global);
   const size_t W = RowUnits(dmax, quads), unit = quads ? 16 : 4, warps = threads / 32;
-  return (global ? 0 : (size_t)dmax * (W | 1) * unit) + warps * (k - 4) * W * unit + (size_t)dmax * 4 +
+  return (global || k == 3 ? 0 : (size_t)dmax * (W | 1) * unit) + warps * (k > 4 ? k - 4 : 0) * W * unit +
+         (size_t)dmax * 4 +
          (global ? 0 : (size_t)6 << TableLg(dmax)) + warps * (k - 3) * (size_t)dmax * 2;
 }
 constexpr size_t CliqueScratchWords(uint32_t dmax) { return (size_t)dmax * (RowUnits(dmax, false) | 1); }
@@ -460,13 +504,14 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
   const uint32_t wcap = RowUnits(dmax, QUADS);
   Unit* sh = reinterpret_cast<Unit*>(cq_sh);
   Unit* mat = GLOBAL ? reinterpret_cast<Unit*>(scratch + (size_t)blockIdx.x * CliqueScratchWords(dmax)) : sh;
-  Unit* sets0 = GLOBAL ? sh : sh + (size_t)dmax * (wcap | 1);
-  Unit* sets = sets0 + (size_t)wid * (K - 4) * wcap;
-  uint32_t* R = reinterpret_cast<uint32_t*>(sets0 + (size_t)WARPS * (K - 4) * wcap);
+  constexpr int kSets = K > 4 ? K - 4 : 0;
+  Unit* sets0 = GLOBAL || K == 3 ? sh : sh + (size_t)dmax * (wcap | 1);
+  Unit* sets = sets0 + (size_t)wid * kSets * wcap;
+  uint32_t* R = reinterpret_cast<uint32_t*>(sets0 + (size_t)WARPS * kSets * wcap);
   const uint32_t tlg = TableLg(dmax);
   uint32_t* keys = R + dmax;
   uint16_t* at = reinterpret_cast<uint16_t*>(keys + (1u << tlg));
-  uint16_t* lists = (GLOBAL ? reinterpret_cast<uint16_t*>(keys) : at + (1u << tlg)) + (size_t)wid * (K - 3) * dmax;
+  uint16_t* lists = (GLOBAL ? reinterpret_cast<uint16_t*>(keys) : at + (1u << tlg)) + (size_t)wid * (K - 3) * dmax;  // K = 3: none
   __shared__ uint32_t s_item, s_row;
   const uint32_t count = min(*nq, cap);
   unsigned long long local = 0, bytes = 0;
@@ -493,28 +538,32 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
     const uint32_t W = RowUnits(d, QUADS), ws = W | 1;
     uint32_t* bits_of = reinterpret_cast<uint32_t*>(mat);  // row i's words start at i * ws * kWords
     for (uint32_t i = tid; i < d; i += THREADS) R[i] = __ldg(L + i);
-    for (uint32_t i = tid; i < d * ws; i += THREADS) mat[i] = RowUnit<QUADS>::Zero();
+    if (K > 3)
+      for (uint32_t i = tid; i < d * ws; i += THREADS) mat[i] = RowUnit<QUADS>::Zero();
     if (!GLOBAL) {
       for (uint32_t i = tid; i < (1u << tlg); i += THREADS) keys[i] = kNoKey;
       __syncthreads();
       for (uint32_t i = tid; i < d; i += THREADS) TablePut(keys, at, tlg, R[i], i);
     }
     __syncthreads();
-    // rows wid, wid + WARPS, ...: the lanes fetch the lists of 32 rows at a
-    // time, then the warp builds them one by one, four loads in flight per
-    // lane (the loads are what a row waits for)
-    for (uint32_t i0 = wid; i0 < d; i0 += WARPS * 32) {
+    // rows wid, wid + WARPS, ... (triangles: of the part's rows, every parts-th
+    // one): the lanes fetch the lists of 32 rows at a time, then the warp
+    // builds them one by one, four loads in flight per lane (the loads are
+    // what a row waits for)
+    const uint32_t row0 = K == 3 ? part : 0, rstep = K == 3 ? parts : 1;
+    const uint32_t nrows = d > row0 ? (d - row0 + rstep - 1) / rstep : 0;
+    for (uint32_t i0 = wid; i0 < nrows; i0 += WARPS * 32) {
       const uint32_t mine = i0 + lane * WARPS;
       const uint32_t* ma = nullptr;
       const uint32_t* mb = nullptr;
       uint32_t mlen = 0;
-      if (mine < d) {
-        CList<ORIENT>(V, R[mine], ma, mlen);
-        if (!ORIENT) mb = HubBitmap(V.G, R[mine]);
+      if (mine < nrows) {
+        CList<ORIENT>(V, R[row0 + mine * rstep], ma, mlen);
+        if (!ORIENT) mb = HubBitmap(V.G, R[row0 + mine * rstep]);
       }
-      const uint32_t rows = min(32u, (d - i0 + WARPS - 1) / WARPS);
+      const uint32_t rows = min(32u, (nrows - i0 + WARPS - 1) / WARPS);
       for (uint32_t k = 0; k < rows; ++k) {
-        const uint32_t i = i0 + k * WARPS;
+        const uint32_t i = row0 + (i0 + k * WARPS) * rstep;
         const uint32_t* a = reinterpret_cast<const uint32_t*>(__shfl_sync(FULL, (unsigned long long)(uintptr_t)ma, k));
         const uint32_t len = __shfl_sync(FULL, mlen, k);
         const uint32_t* bm =
@@ -536,7 +585,8 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
               const unsigned bits = __ballot_sync(FULL, (word[t] >> (x[t] & 31)) & 1u);
-              if (lane == 0 && bits) bits_of[(size_t)i * ws * kWords + (jb >> 5) + t] = bits;  // row i is this warp's
+              if (K == 3) local += lane == 0 ? __popc(bits) : 0;
+              else if (lane == 0 && bits) bits_of[(size_t)i * ws * kWords + (jb >> 5) + t] = bits;  // this warp's row
             }
           }
           if (lane == 0) bytes += 12ULL + 8ULL * (d - i);
@@ -549,7 +599,8 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
               in = pos < len && __ldg(a + pos) == x;
             }
             const unsigned bits = __ballot_sync(FULL, in);
-            if (lane == 0 && bits) bits_of[(size_t)i * ws * kWords + (jb >> 5)] = bits;
+            if (K == 3) local += lane == 0 ? __popc(bits) : 0;
+            else if (lane == 0 && bits) bits_of[(size_t)i * ws * kWords + (jb >> 5)] = bits;
           }
           if (lane == 0) bytes += 12ULL + 8ULL * (d - i);
         } else {
@@ -569,7 +620,8 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
               }
               if (c < d && (ORIENT || c > i)) {
                 const uint32_t lo = min(i, c), hi = max(i, c);
-                atomicOr(bits_of + (size_t)lo * ws * kWords + (hi >> 5), 1u << (hi & 31));
+                if (K == 3) ++local;
+                else atomicOr(bits_of + (size_t)lo * ws * kWords + (hi >> 5), 1u << (hi & 31));
               }
             }
           }
@@ -578,7 +630,7 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
       }
     }
     __syncthreads();
-    while (true) {
+    while (K > 3) {
       uint32_t i = 0;
       if (lane == 0) i = atomicAdd(&s_row, 1u);
       i = __shfl_sync(FULL, i, 0) * parts + part;
@@ -587,8 +639,10 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
       __syncwarp();
       const uint32_t nl = Expand(reinterpret_cast<const uint32_t*>(row), i >> 5, W * kWords, lists);
       __syncwarp();
-      if (nl >= K - 2)
-        local += RowCliques<K - 2, QUADS>(row, lists, nl, mat, ws, W, lists + dmax, dmax, sets, wcap);
+      if constexpr (K > 3)
+        if (nl >= K - 2)
+          local += RowCliques<K - 2, QUADS>(row, lists, nl, mat, ws, W, lists + dmax,
+                                              dmax, sets, wcap);
     }
     __syncthreads();  // the matrix is rebuilt for the next root
   }

@@ -546,7 +546,7 @@ static CountForm FormOf(const sme_opts& o, const Query& q, const Program& p, boo
   if (q.type == 4 && root == 1) return C_HOUSE;
   if (root != 0) return C_STEPS;
   if (q.type == 1) return C_CYCLE4;
-  if (q.n >= 4 && IsOrderedClique(q)) return C_CLIQUE;
+  if (q.n >= 3 && IsOrderedClique(q)) return C_CLIQUE;
   return C_STEPS;
 }
 

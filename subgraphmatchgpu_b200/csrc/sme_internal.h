@@ -243,7 +243,7 @@ struct Step {
 enum CountForm : uint8_t {
   C_STEPS = 0,   // the level program
   C_CYCLE4 = 1,  // Q1: two-path counters (cycle.cuh)
-  C_CLIQUE = 2,  // Q3, Q7, Q11: bit matrices per root (clique.cuh)
+  C_CLIQUE = 2,  // Q0, Q3, Q7, Q11: bit matrices per root (clique.cuh)
   C_HOUSE = 3    // Q4 rooted at u1: two-path counters (house.cuh) less `minus`
 };
 struct Program {

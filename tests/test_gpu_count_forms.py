@@ -83,15 +83,16 @@ def test_graphs_outside_the_contract_keep_the_level_program(resident):
 
 # class edges of the bit matrices: a root of a complete graph of n vertices
 # has n - 1 candidates
-@pytest.mark.parametrize("n,ks", [(4, (4, 5)), (5, (4, 5, 6)), (33, (4, 5, 6)), (34, (4, 5, 6)), (65, (4, 5, 6)),
-                                  (130, (4, 5, 6)), (257, (4, 5)), (258, (4, 5)), (513, (4, 5)), (514, (4,)),
-                                  (1025, (4,)), (1026, (4,))])
+@pytest.mark.parametrize("n,ks", [(2, (3, 4)), (4, (3, 4, 5)), (5, (3, 4, 5, 6)), (33, (3, 4, 5, 6)),
+                                  (34, (3, 4, 5, 6)), (65, (3, 4, 5, 6)), (130, (3, 4, 5, 6)), (257, (3, 4, 5)),
+                                  (258, (3, 4, 5)), (513, (3, 4, 5)), (514, (3, 4)), (1025, (3, 4)), (1026, (3, 4)),
+                                  (1500, (3,))])
 def test_cliques_of_complete_graphs(n, ks):
     g = sme.Graph.clique(n)
     g.to_device(0)
     o, _ = g.degree_order(orient=True)
     for k in ks:
-        q = {4: 3, 5: 7, 6: 11}[k]
+        q = {3: 0, 4: 3, 5: 7, 6: 11}[k]
         assert g.count(q) == comb(n, k)
         assert o.count(q) == comb(n, k)
         # root 0 has n - 1 candidates, root 1 one fewer
@@ -101,7 +102,7 @@ def test_cliques_of_complete_graphs(n, ks):
 # vertex 0 sees every other vertex: a root of d candidates in every class, and
 # above the last one, which keeps the level program
 @pytest.mark.parametrize("d", [31, 256, 257, 700, 896, 897, 960, 961, 1024, 1025, 4096, 4097, 5000])
-@pytest.mark.parametrize("q", [3, 7, 11])
+@pytest.mark.parametrize("q", [0, 3, 7, 11])
 def test_cliques_of_a_hub_root(d, q):
     e = np.concatenate([np.stack([np.zeros(d, np.int64), np.arange(1, d + 1)], 1), 1 + random_edges(d, 14 * d, d)])
     rng = np.random.default_rng(d)
@@ -125,7 +126,7 @@ def test_cliques_of_skewed_graphs(resident):
     renumbered, _ = g.degree_order(orient=False)
     for x in (g, o, renumbered) if resident else ():
         x.to_device(0)
-    for q in (3, 7):
+    for q in (0, 3, 7):
         want = g.count(q, warp_granularity=3)
         assert [x.count(q, a) for x in (g, o, renumbered) for a in ALGOS] == [want] * 9
         part = dict(root_begin=5, root_end=g.n - 9, root_stride=3)
