@@ -2580,9 +2580,9 @@ class Executor {
       }
     }
     Timed t = TimerStart();
-    // the classes are independent: the few large roots (first) run beside the
-    // many small ones on the context's second stream, so neither waits for the
-    // other's last CTAs; a class no list can reach is not launched
+    // the classes are independent: the few large roots (first) and the small
+    // ones run on the context's second stream beside class M, so neither waits
+    // for the other's last CTAs; a class no list can reach is not launched
     constexpr int kWide = K <= 4 ? 1024 : 512;
     const bool fork = bound > kCliqueM;
     if (fork) {
@@ -2593,12 +2593,13 @@ class Executor {
       if (bound > kCliqueL)
         LaunchCliqueClass<K, ORIENT, kWide, false>(V, col, Q, 3, CliqueX(K), nullptr, ctx_.copy_stream);
       LaunchCliqueClass<K, ORIENT, kWide, false>(V, col, Q, 2, kCliqueL, nullptr, ctx_.copy_stream);
-      CK(cudaEventRecord(ctx_.copy_ev[1], ctx_.copy_stream));
     }
     if (bound > kCliqueS)
       LaunchCliqueClass<K, ORIENT, kCliqueMThreads, false>(V, col, Q, 1, kCliqueM, nullptr, st_);
-    k_clique_small<K, ORIENT><<<WarpGrid(P), WARP_BLOCK, 0, st_>>>(V, col, Q.q[0], Q.n, Q.cap[0], ctrl_);
+    k_clique_small<K, ORIENT><<<WarpGrid(P), WARP_BLOCK, 0, fork ? ctx_.copy_stream : st_>>>(V, col, Q.q[0], Q.n,
+                                                                                             Q.cap[0], ctrl_);
     Launched();
+    if (fork) CK(cudaEventRecord(ctx_.copy_ev[1], ctx_.copy_stream));
     if (fork) CK(cudaStreamWaitEvent(st_, ctx_.copy_ev[1], 0));
     TimerStop(t, kPhaseComputeCount);
     if (left) {
