@@ -2158,6 +2158,7 @@ DeviceGraph* UploadGraphToArena(const HostGraph& g, DeviceContext& ctx, uint64_t
   uint64_t bytes = 0;
   std::shared_ptr<const PackedLists> pk = g.packed;
   try {
+    QuiesceOnError quiesce(ctx);
     auto arena_alloc = [&ctx](size_t b) { return ctx.arena.Alloc(b); };
     d->row_ptrs = (uintE*)arena_alloc((g.n + 1) * sizeof(uintE));
     d->cols = (uintV*)arena_alloc(std::max<uint64_t>(g.m, 1) * sizeof(uintV));
@@ -2178,6 +2179,7 @@ DeviceGraph* UploadGraphToArena(const HostGraph& g, DeviceContext& ctx, uint64_t
       FailOnFlag(*reinterpret_cast<const uint32_t*>(ctx.h_pinned));
     }
     CK(cudaStreamSynchronize(ctx.stream));
+    quiesce.done = true;
   } catch (...) {
     delete d;
     throw;
@@ -2267,6 +2269,7 @@ class Executor {
   uint64_t ext_h2d_bytes() const { return ext_bytes_; }
 
   RunResult Run(const RootTask& task) {
+    QuiesceOnError quiesce(ctx_);
     const uint32_t stride = task.stride ? task.stride : 1;
     auto t0 = std::chrono::steady_clock::now();
     size_t mark = A_.Mark();
@@ -2306,6 +2309,7 @@ class Executor {
     unsigned long long h[kCtrl];
     CK(cudaMemcpyAsync(h, ctrl_, sizeof(h), cudaMemcpyDeviceToHost, st_));
     CK(cudaStreamSynchronize(st_));
+    quiesce.done = true;
     float dev_ms = 0;
     cudaEventElapsedTime(&dev_ms, ev0, ev1);
     CK(cudaGetLastError());

@@ -61,6 +61,23 @@ struct DeviceContext {
   ~DeviceContext();
 };
 
+// Leaves nothing of a failed call in flight: a scope left by an exception waits
+// for both streams of the context before the callers above it release the
+// arena, whose bytes the next call writes from either stream (a packed upload
+// starts on the copy stream at once).  `done` is set on the way out of a scope
+// that ended its own work.
+struct QuiesceOnError {
+  DeviceContext& ctx;
+  bool done = false;
+  explicit QuiesceOnError(DeviceContext& c) : ctx(c) {}
+  QuiesceOnError(const QuiesceOnError&) = delete;
+  ~QuiesceOnError() {
+    if (done) return;
+    cudaStreamSynchronize(ctx.stream);
+    cudaStreamSynchronize(ctx.copy_stream);
+  }
+};
+
 // Allocates a context with an arena of `bytes` (0 = most of free memory).
 DeviceContext* CreateContext(int device, uint64_t bytes);
 void DestroyContext(DeviceContext* c);
