@@ -116,6 +116,14 @@ static void CopyInstances(DeviceContext& ctx, void* host, const void* dev, size_
   }
 }
 
+// Gives back what a call took from the arena, however the call ends.
+struct ArenaScope {
+  Arena& arena;
+  const size_t mark;
+  explicit ArenaScope(Arena& a) : arena(a), mark(a.Mark()) {}
+  ~ArenaScope() { arena.Release(mark); }
+};
+
 struct RunOut {
   uint64_t count = 0;
   uint64_t emitted = 0;
@@ -138,6 +146,7 @@ static RunOut Execute(sme_graph* g, const sme_opts& o, bool enumerate, uint32_t*
     slot.bytes = o.mem_limit_bytes;
   }
   DeviceContext& ctx = *slot.ctx;
+  const ArenaScope scope(ctx.arena);
   const RootTask task = TaskOf(o, g->g.n);
   RunResult r;
   uint64_t h2d = 0, d2h = 8;
@@ -148,16 +157,10 @@ static RunOut Execute(sme_graph* g, const sme_opts& o, bool enumerate, uint32_t*
   } else {
     DeviceGraph* dg = g->g.dev;
     bool temp = false;
-    const size_t graph_mark = ctx.arena.Mark();
     if (!dg || dg->device != o.device) {
       // not resident: the graph shares the call's arena (budget covers
       // frontiers + graph) and leaves with it
-      try {
-        dg = UploadGraphToArena(g->g, ctx, &h2d);
-      } catch (...) {
-        ctx.arena.Release(graph_mark);
-        throw;
-      }
+      dg = UploadGraphToArena(g->g, ctx, &h2d);
       temp = true;
     }
     uint32_t* d_out = nullptr;
@@ -187,12 +190,10 @@ static RunOut Execute(sme_graph* g, const sme_opts& o, bool enumerate, uint32_t*
     } catch (...) {
       if (own_out) cudaFree(d_out);
       if (temp) FreeDeviceGraph(dg);
-      ctx.arena.Release(graph_mark);
       throw;
     }
     if (own_out) cudaFree(d_out);
     if (temp) FreeDeviceGraph(dg);
-    ctx.arena.Release(graph_mark);
   }
   if (o.execute_mode != SME_EXTERNAL_GPU) h2d += r.stats.h2d_bytes;  // the root list
   r.stats.h2d_bytes = h2d;

@@ -62,3 +62,18 @@ def test_a_packed_upload_after_a_call_that_ran_out_of_memory(query):
             big.count(query, mem_limit_bytes=budget)
         assert e.value.status == 3  # no room for a level's batch, the ones before it are running
         assert small.count(query, mem_limit_bytes=budget) == want
+
+
+@pytest.mark.gpu
+def test_failed_external_calls_leave_the_arena_as_it_was():
+    # each of them asks for a list cache that the budget cannot hold, after
+    # taking 32 KB for the offsets
+    budget = 1 << 20
+    big, small = sme.Graph.rmat(12, 8, seed=2), sme.Graph.rmat(8, 4, seed=3)
+    rp, cl = small.csr()
+    want = O.count(rp, cl, 3)
+    for _ in range(40):
+        with pytest.raises(sme.SmeError) as e:
+            big.count(3, mode=sme.EXTERNAL_GPU, mem_limit_bytes=budget)
+        assert e.value.status == 3
+    assert small.count(3, mem_limit_bytes=budget) == want
