@@ -2749,17 +2749,27 @@ class Executor {
     ext_bound_ = 0;
   }
 
+  // What a batch of step k may cost at least.  In memory a budget below 1 MiB
+  // is taken for 1 MiB: batches of a few thousand paths cost more launches than
+  // they save memory.  In external mode only while the levels after this one
+  // can take as much: batches there are not held small by the lists they load,
+  // and levels that each took 1 MiB of an arena of a few left none for the
+  // next.  (The last step is a count, which takes next to nothing.)
+  uint64_t AtLeast(size_t k, uint64_t budget) const {
+    uint64_t least = 1 << 20;
+    if (ext_cols_) least = std::min(least, (uint64_t)((double)A_.Free() * 0.85 / (double)((*steps_).size() - k)));
+    return std::max(budget, least);
+  }
+
   // Batch cost of an external step in frontier-budget units: the subgraph
   // bytes count against the list cache (cg scales them so that frontier
   // bytes / budget + list bytes / (cache x ext_overlap_) <= 1).  The list bytes
   // are counted per path, and the paths of a batch share most of their lists,
   // so a batch is first given ext_overlap_ times the cache; one whose lists do
   // not fit after all is halved, and so is the factor.  R-MAT s16, 13 MiB:
-  // 4-cliques 1.07 s in 11 855 batches -> 0.22 s in 2 418.
-  double ExtListCost(uint64_t budget) const {
-    return ext_cols_ && ext_cap_
-               ? 4.0 * (double)std::max<uint64_t>(budget, 1 << 20) / ((double)(ext_cap_ * 4) * ext_overlap_)
-               : 0.0;
+  // 4-cliques 1.07 s in 11 855 batches -> 0.19 s in 2 418.
+  double ExtListCost(size_t k, uint64_t budget) const {
+    return ext_cols_ && ext_cap_ ? 4.0 * (double)AtLeast(k, budget) / ((double)(ext_cap_ * 4) * ext_overlap_) : 0.0;
   }
   std::vector<Timed> events_;  // recorded regions
   double phase_[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -3104,7 +3114,6 @@ class Executor {
   // on the device.
   std::vector<Batch> Batches(const uint64_t* incl, uint32_t P, double pf, double cf, uint64_t budget, Totals t,
                              const uint64_t* incl2 = nullptr, double cg = 0) {
-    budget = std::max<uint64_t>(budget, 1 << 20);
     if (pf * P + cf * (double)t.est + cg * (double)t.lists <= (double)budget)
       return {Batch{0, P, 0, t.est, t.lists}};
     return Split(incl, P, pf, cf, budget, incl2, cg);
@@ -3261,9 +3270,10 @@ class Executor {
         uint64_t* est = (uint64_t*)A_.Alloc((size_t)F.P * 8);
         uint64_t* sd = (uint64_t*)A_.Alloc((size_t)F.P * 8);
         const Totals tot = EstScan<E_LIST>(F, ds, DCond{}, est, sd);
-        const uint64_t bk = Budget(k);
+        // a count takes no memory beyond these two: only its lists are bounded
+        const uint64_t bk = std::max<uint64_t>(Budget(k), 1 << 20);
         const std::vector<Batch> bs =
-            Batches(sd, F.P, 12.0, 0.0, bk, Totals{tot.lists, tot.lists}, sd, ExtListCost(bk));
+            Batches(sd, F.P, 12.0, 0.0, bk, Totals{tot.lists, tot.lists}, sd, ExtListCost(k, bk));
         std::vector<Batch> todo(bs.rbegin(), bs.rend());
         while (!todo.empty()) {
           const Batch b = todo.back();
@@ -3343,7 +3353,7 @@ class Executor {
       TimerStop(to, kPhaseOrganize);
       // child counts of a batch stay within 31-bit path indices
       const uint64_t bk = std::min<uint64_t>(Budget(k), (uint64_t)(cf * 2.0e9));
-      batches = Split(est, F.P, pf, cf, std::max<uint64_t>(bk, 1 << 20));
+      batches = Split(est, F.P, pf, cf, AtLeast(k, bk));
     } else {  // COMPUTE, PATH_COUNT, FILTER
       Timed to = TimerStart();
       est = (uint64_t*)A_.Alloc((size_t)F.P * 8);
@@ -3353,7 +3363,7 @@ class Executor {
       TimerStop(to, kPhaseOrganize);
       const double cf = s.kind == S_PATH_COUNT ? 0 : 4;
       const uint64_t bk = std::min<uint64_t>(Budget(k), (uint64_t)(std::max(cf, 1.0) * 2.0e9));
-      batches = Batches(est, F.P, fixed, cf, bk, t, sumdeg, ExtListCost(bk));
+      batches = Batches(est, F.P, fixed, cf, AtLeast(k, bk), t, sumdeg, ExtListCost(k, bk));
     }
     std::reverse(batches.begin(), batches.end());
     while (!batches.empty()) {
