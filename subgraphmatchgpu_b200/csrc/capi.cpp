@@ -167,9 +167,11 @@ static RunOut Execute(sme_graph* g, const sme_opts& o, bool enumerate, uint32_t*
     bool own_out = false;
     try {
       if (enumerate && cap) {
-        // in the arena when it takes little of it, else an allocation beside it
+        // in the arena when it takes little of one that the engine sized itself
+        // (the budget a caller set is for the graph and the frontiers), else
+        // an allocation beside it
         size_t bytes = (size_t)cap * prog.n * sizeof(uint32_t);
-        if (bytes < ctx.arena.Free() / 8) {
+        if (o.mem_limit_bytes == 0 && bytes < ctx.arena.Free() / 8) {
           d_out = (uint32_t*)ctx.arena.Alloc(bytes);
         } else {
           if (cudaMalloc((void**)&d_out, bytes) != cudaSuccess) {

@@ -1,7 +1,9 @@
 """Calls near the smallest device budget that holds them: a budget that once
 sufficed keeps sufficing."""
+import ctypes as C
 import functools
 
+import numpy as np
 import pytest
 
 import subgraphmatchgpu_b200 as sme
@@ -25,3 +27,16 @@ def test_external_frontiers_leave_room_for_the_next_level(name, query, budget):
     g = graph(name)
     want = g.count(query, warp_granularity=3)
     assert g.count(query, mode=sme.EXTERNAL_GPU, mem_limit_bytes=int(budget * MB)) == want
+
+
+# the buffer for the instances lies beside the budget, not in it: 480 KB of it
+# would be missing from the 4 MiB that these frontiers need
+def test_enumeration_buffers_do_not_take_from_the_budget():
+    g = graph("rmat12")
+    g.to_device(0)
+    want, cap = g.count(3), 30000
+    out, n, o = np.zeros((cap, 4), np.uint32), C.c_uint64(), sme.opts(3, mem_limit_bytes=4 * MB)
+    st = sme.lib().sme_enumerate(g.handle, C.byref(o), out.ctypes.data, cap, C.byref(n))
+    assert (st, n.value) == (8, want), sme.lib().sme_last_error()  # more instances than the buffer holds
+    assert len(np.unique(out, axis=0)) == cap
+    g.release_device()
