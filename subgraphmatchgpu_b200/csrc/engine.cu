@@ -2251,6 +2251,7 @@ class Executor {
   Executor(const Program& prog, const DeviceGraph& g, DeviceContext& ctx, uint32_t* d_out, uint64_t cap)
       : prog_(prog), g_(g), ctx_(ctx), A_(ctx.arena), st_(ctx.stream), out_(d_out), cap_(cap), steps_(&prog.steps) {
     sms_ = SmCount(ctx.device);
+    mat_misses_.assign(std::max(prog.steps.size(), prog.minus.size()), 0);
     lists_simple_ = g.defects >= 0 && !((uint32_t)g.defects & kNotSimple);
   }
 
@@ -2374,6 +2375,9 @@ class Executor {
   uint64_t ext_cap_ = 0, ext_bound_ = 0;
   double ext_overlap_ = 32.0;
   int ext_misses_ = 0;  // counting frontiers whose lists did not fit at once
+  // per step: frontiers whose children did not fit the budget at once, less
+  // those whose children did
+  std::vector<int> mat_misses_;
 
   // The resident graph with its hub bitmaps (`use_bitmaps_` false: lists only).
   DGraph Resident() const {
@@ -3093,15 +3097,20 @@ class Executor {
     else k_scan_add<false, ITEMS><<<nb - 1, SCAN_THREADS, 0, st_>>>(est, nullptr, F.P, bs);
     Launched();
   }
+  // `read`: the totals are wanted (a host round trip; else zeros).
   template <EstKind KIND>
   Totals EstScan(const DFront& F, const DStep& ds, const DCond& dc, uint64_t* est, uint64_t* est2,
-                 uint32_t* first = nullptr) {
+                 uint32_t* first = nullptr, bool read = true) {
     const uint32_t tile = F.P <= kScanSmall ? SCAN_THREADS : SCAN_TILE;
     const uint32_t nb = (F.P + tile - 1) / tile;
     const size_t m = A_.Mark();
     uint64_t* bs = (uint64_t*)A_.Alloc(((size_t)nb + 1) * 16);
     if (tile == SCAN_THREADS) LaunchEstScan<KIND, 1>(F, ds, dc, est, est2, first, nb, bs);
     else LaunchEstScan<KIND, SCAN_ITEMS>(F, ds, dc, est, est2, first, nb, bs);
+    if (!read) {
+      A_.Release(m);
+      return Totals{0, 0};
+    }
     CK(cudaMemcpyAsync(ctx_.h_pinned, bs + nb, 8, cudaMemcpyDeviceToHost, st_));
     if (est2) CK(cudaMemcpyAsync(ctx_.h_pinned + 1, bs + 2 * nb + 1, 8, cudaMemcpyDeviceToHost, st_));
     CK(cudaStreamSynchronize(st_));
@@ -3333,23 +3342,31 @@ class Executor {
       batches.push_back(Batch{0, F.P, 0, 0, 0});
     } else if (s.kind == S_MATERIALIZE) {
       // one batch when all children fit, counted exactly; else batches by the
-      // set sizes, an upper bound, each counted in its turn
-      Timed to = TimerStart();
-      uint64_t* cnt = (uint64_t*)A_.Alloc((size_t)F.P * 8);
-      uint32_t* first = FirstOf(dc, F.P);
-      const Totals t = EstScan<E_CHILD>(F, ds, dc, cnt, nullptr, first);
-      TimerStop(to, kPhaseOrganize);
+      // set sizes, an upper bound, each counted in its turn.  A step that
+      // misses more often than it fits is not tried again: under a small budget
+      // its frontiers would all be counted twice (R-MAT s14, diamonds under 4
+      // MiB by the reuse plan: 6.5 ms without tries, 7.6 with one per frontier,
+      // 6.5 so; 5-cliques under 8 MiB by GPSM, which fit: 35, 22 and 22 ms).
       const double pf = 16, cf = 4.0 * (s.mat_after.size() + s.sets_after.size()) + 16;
-      if (pf * F.P + cf * (double)t.est <= (double)Budget(k) && t.est <= 2000000000ull) {
-        ++batches_;
-        Materialize(k, F, dc, cnt, first, t.est);
+      if (mat_misses_[k] < 3) {
+        Timed to = TimerStart();
+        uint64_t* cnt = (uint64_t*)A_.Alloc((size_t)F.P * 8);
+        uint32_t* first = FirstOf(dc, F.P);
+        const Totals t = EstScan<E_CHILD>(F, ds, dc, cnt, nullptr, first);
+        TimerStop(to, kPhaseOrganize);
+        if (pf * F.P + cf * (double)t.est <= (double)Budget(k) && t.est <= 2000000000ull) {
+          ++batches_;
+          mat_misses_[k] = std::max(mat_misses_[k] - 1, -8);
+          Materialize(k, F, dc, cnt, first, t.est);
+          A_.Release(mark0);
+          return;
+        }
+        ++mat_misses_[k];
         A_.Release(mark0);
-        return;
       }
-      A_.Release(mark0);
       est = (uint64_t*)A_.Alloc((size_t)F.P * 8);
-      to = TimerStart();
-      EstScan<E_SET>(F, ds, dc, est, nullptr);
+      Timed to = TimerStart();
+      EstScan<E_SET>(F, ds, dc, est, nullptr, nullptr, false);
       TimerStop(to, kPhaseOrganize);
       // child counts of a batch stay within 31-bit path indices
       const uint64_t bk = std::min<uint64_t>(Budget(k), (uint64_t)(cf * 2.0e9));

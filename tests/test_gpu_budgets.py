@@ -40,3 +40,16 @@ def test_enumeration_buffers_do_not_take_from_the_budget():
     assert (st, n.value) == (8, want), sme.lib().sme_last_error()  # more instances than the buffer holds
     assert len(np.unique(out, axis=0)) == cap
     g.release_device()
+
+
+# a materialising step whose frontiers never fit at once counts their children
+# once per batch, not once more per frontier
+def test_frontiers_that_never_fit_are_not_counted_twice():
+    g = graph("rmat14")
+    g.to_device(0)
+    want = g.count(2, warp_granularity=3)
+    assert g.count(2, sme.GPU_GPSM_REUSE, mem_limit_bytes=4 * MB) == want
+    s = sme.last_stats()
+    assert s.batches > 50
+    assert s.kernel_launches < 5 * s.batches  # 366 for 78 batches; 394 with a count per frontier
+    g.release_device()
