@@ -786,6 +786,38 @@ void LaunchRun(sme_batch_plan* p) {
   if (p->ncycle) BCK(cudaStreamWaitEvent(p->stream, p->join, 0));
 }
 
+// Whether the 4-cycles of a graph go through k_batch_cycle.  Up to kCycleSpan
+// vertices, one range of counters a root, they always do.  Every range costs a
+// root's warp its clearing and a search in each neighbour's list, about 0.1 ns
+// of the device and 0.08 a neighbour (1 us and 0.1 of the one warp), the
+// depth-first kernel 0.17 ns an element of the neighbours' lists (1 us of one
+// group), of the neighbours above the root in both: the many small roots of a
+// large flat graph are better off depth first, its largest root decides where
+// there are hubs.  Alone in a batch, counters and depth first: flat graphs of
+// degree 4 with 2^16, 2^17, 2^18 and 2^20 vertices 0.21 and 0.28, 0.67 and
+// 0.37, 2.4 and 0.50, 33.8 and 1.9 ms; of degree 16 with 2^17 and 2^18 1.8 and
+// 3.6, 7.0 and 6.3; Barabasi-Albert, 2^18 vertices of 4 edges, 9.5 and 107.
+bool CountersPay(const HostGraph& g) {
+  if (g.n <= kCycleSpan) return true;
+  double counters = 0, dfs = 0, counters_most = 0, dfs_most = 0;
+  for (uint64_t u = 0; u < g.n; ++u) {
+    double above = 0, elems = 0;
+    for (uint64_t j = g.row_ptrs[u]; j < g.row_ptrs[u + 1]; ++j) {
+      const uintV v = g.cols[j];
+      if (v <= u) continue;
+      above += 1;
+      elems += (double)(g.row_ptrs[v + 1] - g.row_ptrs[v]);
+    }
+    if (above < 2) continue;  // no cycle: neither kernel looks further
+    const double ranges = (double)((g.n - 1 - u + kCycleSpan - 1) / kCycleSpan);
+    counters += ranges * (0.1 + 0.08 * above);
+    counters_most = std::max(counters_most, 1000 * ranges * (1 + 0.1 * above));
+    dfs += 0.17 * elems;
+    dfs_most = std::max(dfs_most, 1000 * elems);
+  }
+  return std::max(dfs, dfs_most) >= std::max(counters, counters_most);
+}
+
 // The graph's contract for the two other ways: strictly increasing lists
 // without the vertex itself, every edge in both directions.  Vertices are
 // visited in order, so u is the next unread element of each of its
@@ -852,7 +884,8 @@ void Prepare(sme_graph* const* graphs, const int32_t* queries, uint64_t num, con
     const int q = qs[i];
     const bool clique = q == 0 || q == 3 || q == 7 || q == 11;
     const bool other_way = !g.oriented && (clique || q == 1) && SimpleSymmetric(g, cursor);
-    const bool orient = other_way && clique, cycle = other_way && q == 1 && g.MaxDegree() <= 0xFFFFu;
+    const bool orient = other_way && clique;
+    const bool cycle = other_way && q == 1 && g.MaxDegree() <= 0xFFFFu && CountersPay(g);
     qv[i] = (uint8_t)(orient ? kOrientedProg + q : q);
     qs[i] = qv[i];
     uint64_t base = cols.size();

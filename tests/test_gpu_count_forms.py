@@ -169,6 +169,23 @@ def test_batched_cycles_and_cliques():
     assert only.run()[0].tolist() == want[:1]
 
 
+# a large flat graph: its roots' few two-paths are not worth a pass over every
+# range of counters (the same graph with a loop is always searched depth first)
+def test_batched_cycles_of_a_large_flat_graph():
+    n = 1 << 19
+    e = random_edges(n, 2 * n, 11)
+    ms, counts = [], []
+    for extra in ([], [(n, n)]):
+        g = sme.Graph.from_csr(*csr_of(n + 1, np.concatenate([e, extra]) if extra else e))
+        plan = sme.BatchPlan([g], [1])
+        runs = [plan.run() for _ in range(7)]
+        counts += [int(c[0]) for c, _ in runs]
+        ms.append(min(t for _, t in runs))
+        plan.close()
+    assert counts == [g.count(1, warp_granularity=1)] * 14
+    assert ms[0] < 2.5 * ms[1]
+
+
 @pytest.mark.parametrize("n", [5, 12, 20, 65, 130])
 def test_houses_of_complete_graphs(n):
     g = sme.Graph.clique(n)
