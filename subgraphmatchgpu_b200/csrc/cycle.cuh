@@ -239,6 +239,17 @@ __device__ __forceinline__ uint64_t CtaInclusive(uint64_t v, uint64_t* wtot) {
   return v + (wid ? wtot[wid - 1] : 0);
 }
 
+// A range costs a CTA its clearing and two searches in every neighbour's list,
+// 50 ns of the device and 0.31 a neighbour, a two-path of the level program
+// 0.42 ns and more (trees under 64 and 512 roots with 10, 100 and 300
+// neighbours in graphs of 2^18 to 2^25 vertices).  A root whose two-paths are
+// fewer than its ranges ask for goes to `left`, which the level program takes:
+// 512 roots of 30 000 two-paths and 300 neighbours each, 2^25 vertices, 24.1
+// ms by counters, 5.1 by the level program; 2^22 vertices 2.1 and 5.
+__device__ __forceinline__ bool RangesPay(uint64_t two_paths, uint32_t ranges, uint32_t d) {
+  return ranges == 1 || two_paths >= (uint64_t)ranges * (128 + 3ull * d / 4);
+}
+
 // Entries of `tiles`: queued root index << 32 | range.
 template <bool TILED>
 __global__ void __launch_bounds__(CYC_THREADS, 1) k_cycle4_cta(DGraph G, uint32_t n,
@@ -246,7 +257,8 @@ __global__ void __launch_bounds__(CYC_THREADS, 1) k_cycle4_cta(DGraph G, uint32_
                                                                const uint32_t* __restrict__ queue,
                                                                const uint32_t* __restrict__ nqueue, uint32_t* next,
                                                                uint64_t* tiles, uint32_t* ntiles, uint32_t tiles_cap,
-                                                               uint32_t* err, unsigned long long* acc) {
+                                                               uint32_t* left, uint32_t* nleft, uint32_t* err,
+                                                               unsigned long long* acc) {
   extern __shared__ uint64_t cyc_sh[];
   uint64_t* off = cyc_sh;                 // exclusive offsets of the chunk's lists, then their sum
   uint64_t* ptr = off + CYC_THREADS + 2;  // first element of each (16-byte aligned, as is the table)
@@ -292,8 +304,11 @@ __global__ void __launch_bounds__(CYC_THREADS, 1) k_cycle4_cta(DGraph G, uint32_
       if (total > kCycleHashMax) {
         const uint32_t ranges = (uint32_t)((n - 1 - (uint64_t)u0 + tile - 1) / tile);
         if (tid == 0) {
-          const uint32_t at = atomicAdd(ntiles, ranges);
-          for (uint32_t k = 0; k < ranges; ++k)
+          const bool pay = RangesPay(total, ranges, d);
+          if (!pay) left[atomicAdd(nleft, 1u)] = u0;  // a queued root once at most
+          const uint32_t count = pay ? ranges : 0;
+          const uint32_t at = atomicAdd(ntiles, count);
+          for (uint32_t k = 0; k < count; ++k)
             if (at + k < tiles_cap) tiles[at + k] = (uint64_t)slot << 32 | k;
             else atomicOr(err, ENGINE_ERR_BOUNDS);
         }

@@ -2304,12 +2304,21 @@ class Executor {
       F.inst[s0.u] = col;
       ++batches_;
       if (!CountByForm(task, col, P)) Level(1, F);
+      if (i0 + P >= nroots) break;  // what the last chunk left is told by the final read
+      if (left_) RunLeft((uint32_t)ReadU64((const uint64_t*)(ctrl_ + 14)));
       A_.Release(m);
     }
-    CK(cudaEventRecord(ev1, st_));
     unsigned long long h[kCtrl];
-    CK(cudaMemcpyAsync(h, ctrl_, sizeof(h), cudaMemcpyDeviceToHost, st_));
-    CK(cudaStreamSynchronize(st_));
+    auto finish = [&] {
+      CK(cudaEventRecord(ev1, st_));
+      CK(cudaMemcpyAsync(h, ctrl_, sizeof(h), cudaMemcpyDeviceToHost, st_));
+      CK(cudaStreamSynchronize(st_));
+    };
+    finish();
+    if (h[14]) {
+      RunLeft((uint32_t)h[14]);
+      finish();
+    }
     quiesce.done = true;
     float dev_ms = 0;
     cudaEventElapsedTime(&dev_ms, ev0, ev1);
@@ -2361,10 +2370,11 @@ class Executor {
   bool lists_simple_ = false;  // known to hold no element twice
   // [0] count [1] bytes [3] error flags [4] list cache overflow
   // [5] reuse hits [6] list cache elements [7] ticket of k_est_scan; [8..13]
-  // count, bytes and hits of Program::minus
+  // count, bytes and hits of Program::minus [14] roots in left_
   static constexpr int kCtrl = 16;
   unsigned long long* ctrl_ = nullptr;
   unsigned long long* acc_ = nullptr;  // counters of the program being run
+  uint32_t* left_ = nullptr;           // roots that CountCycles leaves to the steps
   uint64_t emitted_ = 0;               // instances written (or counted past the capacity)
   uint64_t minus_paths_ = 0;           // paths of the last step of Program::minus
   uint64_t launches_ = 0, batches_ = 0, paths_ = 0, hot_ = 0, root_h2d_ = 0;
@@ -2378,6 +2388,16 @@ class Executor {
   // per step: frontiers whose children did not fit the budget at once, less
   // those whose children did
   std::vector<int> mat_misses_;
+
+  // The steps over the roots left_[0..n).
+  void RunLeft(uint32_t n) {
+    DFront F{};
+    F.P = n;
+    F.inst[(*steps_)[0].u] = left_;
+    left_ = nullptr;
+    CK(cudaMemsetAsync(ctrl_ + 14, 0, sizeof(unsigned long long), st_));
+    Level(1, F);
+  }
 
   // The resident graph with its hub bitmaps (`use_bitmaps_` false: lists only).
   DGraph Resident() const {
@@ -2628,7 +2648,9 @@ class Executor {
     // which a graph of 65536 vertices or fewer never needs)
     const uint64_t per = kCycleTable / (g_.n > 0xFFFFu ? 4 : 2);
     const uint64_t ranges = (g_.n + per - 1) / per;
-    if (P * ranges > 0xFFFFFFFFull || P * (ranges * 8 + 4) > A_.Free() / 2) return false;
+    if (P * ranges > 0xFFFFFFFFull || P * (ranges * 8 + 8) > A_.Free() / 2) return false;
+    left_ = (uint32_t*)A_.Alloc((size_t)P * 4);  // released with the chunk of roots
+    uint32_t* nleft = (uint32_t*)(ctrl_ + 14);
     const size_t mark = A_.Mark();
     static std::atomic<bool> set[64];  // per device, once (twice is harmless)
     const int dv = ctx_.device;
@@ -2651,15 +2673,15 @@ class Executor {
     const unsigned ctas = (unsigned)std::min<uint64_t>(sms_, P);
     k_cycle4_warp<<<grid, CYW_THREADS, kCycleWarpSmem, st_>>>(G, col, P, ctl, queue, ctl + 1, ctrl_);
     k_cycle4_cta<false><<<ctas, CYC_THREADS, kCycleCtaSmem, st_>>>(G, (uint32_t)g_.n, col, queue, ctl + 1, ctl + 2,
-                                                                    tiles, ctl + 3, (uint32_t)(P * ranges), err,
-                                                                    ctrl_);
+                                                                    tiles, ctl + 3, (uint32_t)(P * ranges), left_,
+                                                                    nleft, err, ctrl_);
     launches_ += 2;
     // more two-paths than the table takes need more than kCycleHashMax edges
     if (g_.m > kCycleHashMax) {
       const unsigned most = (unsigned)std::min<uint64_t>(sms_, (uint64_t)P * ranges);
       k_cycle4_cta<true><<<most, CYC_THREADS, kCycleCtaSmem, st_>>>(G, (uint32_t)g_.n, col, queue, ctl + 1, ctl + 4,
-                                                                     tiles, ctl + 3, (uint32_t)(P * ranges), err,
-                                                                     ctrl_);
+                                                                     tiles, ctl + 3, (uint32_t)(P * ranges), left_,
+                                                                     nleft, err, ctrl_);
       ++launches_;
     }
     TimerStop(t, kPhaseComputeCount);

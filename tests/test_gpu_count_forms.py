@@ -50,6 +50,50 @@ def test_cycles_over_several_counter_ranges(leaves):
     assert g.count(1) == 3 * (leaves * (leaves - 1) // 2)
 
 
+def tree_with_closures(n, mids, leaves, seed):
+    """Vertex 0 with `mids` neighbours, each with `leaves` more of the n, a few
+    of them shared."""
+    rng = np.random.default_rng(seed)
+    mid = np.arange(1, mids + 1)
+    far = rng.integers(mids + 1, n, mids * leaves)
+    far[:: leaves // 2] = rng.choice(far, len(far[:: leaves // 2]))
+    return np.concatenate([np.stack([np.zeros(mids, np.int64), mid], 1), np.stack([np.repeat(mid, leaves), far], 1)])
+
+
+# a root above the hash table whose two-paths are worth its ranges of counters,
+# and one whose are not: 100 ranges, 300 neighbours, about 35 000 two-paths
+# asked for (paths_processed: the root alone, or the level program's paths too)
+@pytest.mark.parametrize("mids,leaves,counters", [(300, 90, False), (300, 112, False), (300, 125, True), (300, 200, True),
+                                                  (100, 250, True)])
+def test_cycles_of_a_root_with_few_two_paths_for_its_ranges(mids, leaves, counters):
+    n = 100 * 98304 + 1
+    g = sme.Graph.from_csr(*csr_of(n, tree_with_closures(n, mids, leaves, leaves)))
+    g.to_device(0)
+    want = g.count(1, roots=[0], warp_granularity=3)
+    assert want > 0
+    assert g.count(1, roots=[0]) == want
+    assert (sme.last_stats().paths_processed == 1) == counters
+    assert g.count(1, roots=[0, 5, 0]) == 2 * want + g.count(1, roots=[5], warp_granularity=3)
+
+
+def test_roots_left_by_several_chunks_of_a_task():
+    # a task cut into chunks by an 80 MiB budget; every chunk leaves some roots
+    # (8000 neighbours, 25 600 two-paths, five ranges) to the level program
+    n, mids = 400000, 8000
+    rng = np.random.default_rng(1)
+    e = np.concatenate([np.stack([np.zeros(mids, np.int64), np.arange(1, mids + 1)], 1),
+                        np.stack([rng.integers(1, mids + 1, 26500), rng.integers(mids + 1, n, 26500)], 1)])
+    g = sme.Graph.from_csr(*csr_of(n, e))
+    g.to_device(0)
+    want = g.count(1, roots=[0], warp_granularity=3)
+    roots = np.full(1200000, n - 1, np.uint32)
+    roots[[7, 500000, 500001, 900000, 1199999]] = 0
+    assert g.count(1, roots=[n - 1]) == 0
+    assert g.count(1, roots=roots, mem_limit_bytes=80 << 20) == 5 * want
+    s = sme.last_stats()
+    assert s.batches >= 3 and s.paths_processed > len(roots) + 5 * 8000
+
+
 @pytest.mark.parametrize("scale,ef", [(8, 4), (11, 9), (13, 8)])
 def test_cycles_match_oracle_and_level_program(scale, ef):
     g = sme.Graph.rmat(scale, ef, seed=scale)
