@@ -2368,6 +2368,7 @@ class Executor {
   const std::vector<Step>* steps_;  // the level program being run
   int sms_ = 148;
   bool lists_simple_ = false;  // known to hold no element twice
+  int verdict_[2] = {-1, -1};  // Defects without and with symmetry, -1 not asked
   // [0] count [1] bytes [3] error flags [4] list cache overflow
   // [5] reuse hits [6] list cache elements [7] ticket of k_est_scan; [8..13]
   // count, bytes and hits of Program::minus [14] roots in left_
@@ -2406,17 +2407,19 @@ class Executor {
   }
 
   // k_check_simple's verdict on the graph (found at upload for a resident
-  // one, else here).
+  // one, else here, once per call; one on symmetry is one on the lists too).
   uint32_t Defects(bool sym) {
     if (g_.defects >= 0) return (uint32_t)g_.defects;
+    if (verdict_[1] >= 0) return (uint32_t)verdict_[1];
+    if (!sym && verdict_[0] >= 0) return (uint32_t)verdict_[0];
     const size_t mark = A_.Mark();
     uint32_t* flag = (uint32_t*)A_.Alloc(sizeof(uint32_t));
     CK(cudaMemsetAsync(flag, 0, sizeof(uint32_t), st_));
     LaunchCheck(g_, sym, flag, st_);
     Launched();
-    const uint32_t r = (uint32_t)ReadU32(flag);
+    verdict_[sym] = (int)ReadU32(flag);
     A_.Release(mark);
-    return r;
+    return (uint32_t)verdict_[sym];
   }
 
   // Counts the roots col[0..P) with the program's own kernel when it has one
@@ -2434,6 +2437,7 @@ class Executor {
     if (prog_.form == C_CYCLE4) return !Defects(true) && CountCycles(col, P);
     if (prog_.form == C_HOUSE) return !Defects(true) && CountHouses(col, P);
     const bool all = !task.list && task.begin == 0 && task.end >= g_.n && task.stride <= 1 && P == g_.n;
+    if (prog_.n == 3 && (!all || oriented_)) return false;  // (see below): no need to ask
     const uint32_t bad = Defects(all && !oriented_);
     if (bad & kNotSimple) return false;
     const bool orient = all && !oriented_ && !(bad & kNotSymmetric) && g_.m / 2 < 0xFFFFFFFFull;

@@ -125,6 +125,29 @@ def test_graphs_outside_the_contract_keep_the_level_program(resident):
             assert g.count(q) == g.count(q, warp_granularity=1), q
 
 
+def launches(g, q, want, **kw):
+    assert g.count(q, **kw) == want
+    return sme.last_stats().kernel_launches
+
+
+# a graph that comes with the call is checked in it: once however many chunks
+# its task is cut into, and not at all where the answer changes nothing
+def test_the_check_of_a_graph_that_is_not_resident():
+    g = sme.Graph.rmat(10, 8, seed=6)
+    o, _ = g.degree_order(orient=True)
+    roots = np.full(1200000, g.n - 1, np.uint32)  # three chunks under 80 MiB
+    tasks = [(g, 0, dict(roots=np.arange(0, g.n, 2)), 0), (g, 0, dict(root_begin=1), 0), (o, 0, dict(), 0),
+             (g, 0, dict(), 1), (g, 3, dict(roots=np.arange(0, g.n, 2)), 1),
+             (g, 1, dict(roots=roots, mem_limit_bytes=80 << 20), 1)]
+    wants = [x.count(q, warp_granularity=2 if x.oriented else 3, **kw) for x, q, kw, _ in tasks]
+    per_call = [launches(x, q, w, **kw) for (x, q, kw, _), w in zip(tasks, wants)]
+    for x in (g, o):
+        x.to_device(0)
+    resident = [launches(x, q, w, **kw) for (x, q, kw, _), w in zip(tasks, wants)]
+    assert sme.last_stats().batches >= 3
+    assert [a - b for a, b in zip(per_call, resident)] == [c for *_, c in tasks]
+
+
 # class edges of the bit matrices: a root of a complete graph of n vertices
 # has n - 1 candidates
 @pytest.mark.parametrize("n,ks", [(2, (3, 4)), (4, (3, 4, 5)), (5, (3, 4, 5, 6)), (33, (3, 4, 5, 6)),
