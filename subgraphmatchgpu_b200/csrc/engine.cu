@@ -1835,18 +1835,16 @@ void BuildHubRange(const DeviceGraph* d, const HubPlan& hp, uint32_t first, uint
   }
 }
 
-// Plan + build of every hub, synchronised.  `scratch_owned` frees the hub
-// list afterwards (cudaMalloc'd).  Returns the host->device bytes.
+// Plan + build of every hub, queued on `stream`: the caller keeps the plan (the
+// hub list is copied from it) until it has waited for the stream.  Returns the
+// host->device bytes.
 template <typename Alloc>
-uint64_t BuildHubBitmaps(DeviceGraph* d, const HostGraph& g, cudaStream_t stream, Alloc alloc, bool scratch_owned,
-                         uint64_t room) {
-  HubPlan hp;
-  if (!PlanHubBitmaps(d, g, stream, alloc, room, &hp)) return 0;
-  BuildHubRange(d, hp, 0, (uint32_t)hp.hubs().size(), stream);
-  CK(cudaStreamSynchronize(stream));
+uint64_t BuildHubBitmaps(DeviceGraph* d, const HostGraph& g, cudaStream_t stream, Alloc alloc, uint64_t room,
+                         HubPlan* hp) {
+  if (!PlanHubBitmaps(d, g, stream, alloc, room, hp)) return 0;
+  BuildHubRange(d, *hp, 0, (uint32_t)hp->hubs().size(), stream);
   CK(cudaGetLastError());
-  if (scratch_owned) cudaFree(hp.d_hubs);
-  return (uint64_t)hp.hubs().size() * 4;
+  return (uint64_t)hp->hubs().size() * 4;
 }
 
 // ------------------------------------------------------------ packed lists --
@@ -2100,6 +2098,7 @@ DeviceGraph* UploadGraph(const HostGraph& g, int device, cudaStream_t stream, ui
   uint64_t bytes = 0;
   std::shared_ptr<const PackedLists> pk = g.packed;
   uint8_t* scratch = nullptr;
+  HubPlan hp;
   try {
     // one word after the row pointers for k_check_simple's flag
     CK(cudaMalloc((void**)&d->row_ptrs, (g.n + 2) * sizeof(uintE)));
@@ -2120,7 +2119,6 @@ DeviceGraph* UploadGraph(const HostGraph& g, int device, cudaStream_t stream, ui
     } else {
       CK(cudaMemcpyAsync(d->row_ptrs, g.row_ptrs, (g.n + 1) * sizeof(uintE), cudaMemcpyHostToDevice, stream));
       if (g.m) CK(cudaMemcpyAsync(d->cols, g.cols, g.m * sizeof(uintV), cudaMemcpyHostToDevice, stream));
-      CK(cudaStreamSynchronize(stream));
       bytes = (g.n + 1) * sizeof(uintE) + g.m * sizeof(uintV);
     }
     auto dev_alloc = [](size_t b) {
@@ -2130,17 +2128,20 @@ DeviceGraph* UploadGraph(const HostGraph& g, int device, cudaStream_t stream, ui
     };
     size_t fr = 0, tot = 0;
     CK(cudaMemGetInfo(&fr, &tot));
-    bytes += BuildHubBitmaps(d, g, stream, dev_alloc, true, fr);
+    bytes += BuildHubBitmaps(d, g, stream, dev_alloc, fr, &hp);
     uint32_t* flag = reinterpret_cast<uint32_t*>(d->row_ptrs + g.n + 1);
     CK(cudaMemsetAsync(flag, 0, sizeof(uint32_t), stream));
     LaunchCheck(*d, true, flag, stream);
     uint32_t defects = 0;
     CK(cudaMemcpyAsync(&defects, flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-    CK(cudaStreamSynchronize(stream));
+    CK(cudaStreamSynchronize(stream));  // the upload's only wait (a packed one has another)
     CK(cudaGetLastError());
     d->defects = (int)defects;
+    if (hp.d_hubs) cudaFree(hp.d_hubs);
   } catch (...) {
+    cudaStreamSynchronize(stream);  // copies and kernels on the arrays freed below
     if (scratch) cudaFree(scratch);
+    if (hp.d_hubs) cudaFree(hp.d_hubs);
     FreeDeviceGraph(d);
     throw;
   }
@@ -2157,6 +2158,7 @@ DeviceGraph* UploadGraphToArena(const HostGraph& g, DeviceContext& ctx, uint64_t
   d->in_arena = true;
   uint64_t bytes = 0;
   std::shared_ptr<const PackedLists> pk = g.packed;
+  HubPlan hp;
   try {
     QuiesceOnError quiesce(ctx);
     auto arena_alloc = [&ctx](size_t b) { return ctx.arena.Alloc(b); };
@@ -2171,7 +2173,7 @@ DeviceGraph* UploadGraphToArena(const HostGraph& g, DeviceContext& ctx, uint64_t
       CK(cudaMemcpyAsync(d->row_ptrs, g.row_ptrs, (g.n + 1) * sizeof(uintE), cudaMemcpyHostToDevice, ctx.stream));
       if (g.m) CK(cudaMemcpyAsync(d->cols, g.cols, g.m * sizeof(uintV), cudaMemcpyHostToDevice, ctx.stream));
       bytes = (g.n + 1) * sizeof(uintE) + g.m * sizeof(uintV);
-      bytes += BuildHubBitmaps(d, g, ctx.stream, arena_alloc, false, ctx.arena.Free());
+      bytes += BuildHubBitmaps(d, g, ctx.stream, arena_alloc, ctx.arena.Free(), &hp);
     }
     if (flag) {
       CK(cudaMemcpyAsync(ctx.h_pinned, flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx.stream));
