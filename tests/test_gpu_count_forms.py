@@ -2,6 +2,9 @@
 cliques on bit matrices)
 against the oracle, closed forms and the level program (an explicit launch
 shape keeps the level program)."""
+import os
+import subprocess
+import sys
 from math import comb
 
 import numpy as np
@@ -309,3 +312,24 @@ def test_enumeration_over_several_staging_halves():
     inst = g.enumerate(3)
     key = np.sort(inst.astype(np.int64) @ [216000, 3600, 60, 1])
     assert len(np.unique(key)) == comb(60, 4) == len(inst)
+
+
+def test_staging_takes_no_more_threads_than_the_process_may_use():
+    code = """
+import os, sys
+os.sched_setaffinity(0, {sorted(os.sched_getaffinity(0))[0]})
+sys.path.insert(0, sys.argv[1])
+import subgraphmatchgpu_b200 as sme
+threads = lambda: len(os.listdir("/proc/self/task"))
+g = sme.Graph.clique(60)
+g.enumerate(0)  # 410 KB: a plain copy
+before = threads()
+assert len(g.enumerate(3)) == 487635  # 7.8 MB: staged
+print(before, threads())
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = {k: v for k, v in os.environ.items() if not k.startswith("OMP")}
+    r = subprocess.run([sys.executable, "-c", code, root], capture_output=True, text=True, timeout=300, env=env)
+    assert r.returncode == 0, r.stderr
+    before, after = map(int, r.stdout.split())
+    assert after == before
