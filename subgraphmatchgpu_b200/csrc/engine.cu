@@ -2431,11 +2431,13 @@ class Executor {
   bool CountByForm(const RootTask& task, const uint32_t* col, uint32_t P) {
     if (prog_.form == C_STEPS || ext_cols_ || g_.n > 0xFFFFFFFEu || A_.Free() < kFormArena + (uint64_t)P * 8)
       return false;
-    // a graph that came with the call is checked in it, which costs 26 ps an
-    // edge (0.83 ms on R-MAT s20); a root's level program costs about 6 us for
-    // the 4-cycle and the house, 55 ns for the cliques: few roots of a large
-    // graph keep it
-    if (g_.defects < 0 && (uint64_t)P << (prog_.form == C_CLIQUE ? 14 : 17) < g_.m) return false;
+    // a graph that came with the call is checked in it: 3.6 ps an edge for the
+    // lists, 28 with symmetry, and a host round trip (R-MAT s20: 0.11 and 0.88
+    // ms of kernel).  A root saves 20 ns of the 4-clique's level program (0.66
+    // ms for 16 384 roots, 0.26 on the matrices; 85 ns for 5-cliques) and 6 us
+    // of the 4-cycle's and the house's: few roots of a large graph keep it
+    // (2 000 roots of R-MAT s20: 0.26 ms, 0.31 with the check; 4 000: equal)
+    if (g_.defects < 0 && (uint64_t)P * (prog_.form == C_CLIQUE ? 6000 : 1 << 17) < g_.m) return false;
     if (prog_.form == C_CYCLE4) return !Defects(true) && CountCycles(col, P);
     if (prog_.form == C_HOUSE) return !Defects(true) && CountHouses(col, P);
     const bool all = !task.list && task.begin == 0 && task.end >= g_.n && task.stride <= 1 && P == g_.n;

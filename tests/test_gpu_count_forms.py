@@ -151,6 +151,18 @@ def test_the_check_of_a_graph_that_is_not_resident():
     assert [a - b for a, b in zip(per_call, resident)] == [c for *_, c in tasks]
 
 
+# clique roots are worth the check of the lists from one in 6000 edges on
+# (paths_processed counts the roots where the matrices take them)
+def test_few_clique_roots_of_a_large_graph_that_is_not_resident():
+    g = sme.Graph.rmat(14, 12, seed=2)
+    least = -(-g.m // 6000)
+    for count in (least - 1, least):
+        roots = np.arange(count, dtype=np.uint32)
+        want = g.count(3, roots=roots, warp_granularity=3)
+        assert g.count(3, roots=roots) == want
+        assert (sme.last_stats().paths_processed == count) == (count == least)
+
+
 # class edges of the bit matrices: a root of a complete graph of n vertices
 # has n - 1 candidates
 @pytest.mark.parametrize("n,ks", [(2, (3, 4)), (4, (3, 4, 5)), (5, (3, 4, 5, 6)), (33, (3, 4, 5, 6)),
