@@ -45,14 +45,16 @@ def s20():
 
 
 def run_all(g, q, want, **task):
-    """Every plan in memory, and LIGHT in external mode (the only plan the
+    """Every plan in memory, as it runs by default and its level program (kept
+    by granularity 3), and LIGHT in external mode (the only plan the
     external mode runs), on the same task.  A task's roots are the vertices
     of the plan's first pattern vertex: u0 in every plan but the LIGHT house
     (Q4), which starts at u1 (its search sequence is 1 2 3 0 4), so for Q4
     only the plans rooted at u0 count the oracle's task."""
     for algo in (PLANS if q != 4 else (sme.GPU_GPSM, sme.GPU_GPSM_REUSE)):
-        got = g.count(q, algo, **task)
-        assert got == want, (q, algo, task.get("root_begin"), got, want)
+        for gran in (0, 3):
+            got = g.count(q, algo, warp_granularity=gran, **task)
+            assert got == want, (q, algo, gran, task.get("root_begin"), got, want)
     if q == 4:
         return
     got = g.count(q, sme.GPU_LIGHT, mode=sme.EXTERNAL_GPU, **task)
@@ -114,10 +116,18 @@ def test_explicit_root_task_counts_each_listed_root():
 def test_count_steps_grouped_by_hub(monkeypatch):
     # SME_GROUP_BY_HUB=1: a count step takes its paths grouped by the hub
     # whose bitmap it probes (a counting sort of the frontier); the count is
-    # the same in any order
+    # the same in any order.  The explicit launch shape keeps the level
+    # programs, whose last steps these are: one list and a cached set, two
+    # lists, three lists; the grouping shows as launches of its own
     g, _ = engine_graph(16, 16)
-    want = {q: g.count(q, sme.GPU_LIGHT) for q in (3, 2, 1)}
+    cases = [(q, a) for q in (3, 2, 1) for a in (sme.GPU_LIGHT, sme.GPU_GPSM)]
+    want, plain = {}, {}
+    for q, a in cases:
+        want[q, a] = g.count(q, a, warp_granularity=3)
+        plain[q, a] = sme.last_stats().kernel_launches
     monkeypatch.setenv("SME_GROUP_BY_HUB", "1")
-    for q, w in want.items():
-        assert g.count(q, sme.GPU_LIGHT) == w, q
-        assert g.count(q, sme.GPU_GPSM) == w, q
+    for q, a in cases:
+        assert g.count(q, a, warp_granularity=3) == want[q, a] == want[q, sme.GPU_GPSM], (q, a)
+        grouped = sme.last_stats().kernel_launches
+        # the diamond's LIGHT plan has a path count, which is not grouped
+        assert (grouped > plain[q, a]) == ((q, a) != (2, sme.GPU_LIGHT)), (q, a, plain[q, a], grouped)

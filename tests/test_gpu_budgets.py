@@ -29,6 +29,17 @@ def test_external_frontiers_leave_room_for_the_next_level(name, query, budget):
     assert g.count(query, mode=sme.EXTERNAL_GPU, mem_limit_bytes=int(budget * MB)) == want
 
 
+# paths that share next to no lists: a batch sized for 32 times the list cache
+# (3 of 12.8 MB) does not fit it and is halved until it does, again and again
+@pytest.mark.parametrize("query", [0, 3])
+def test_external_batches_whose_lists_do_not_fit_are_halved(query):
+    g = sme.Graph.er(200000, 16.0, seed=9)
+    want = g.count(query, warp_granularity=3)
+    assert g.count(query, mode=sme.EXTERNAL_GPU, mem_limit_bytes=8 * MB) == want
+    s = sme.last_stats()
+    assert s.batches > 8 and s.h2d_bytes > 8 * (g.n + 1) + 4 * g.m  # lists came more than once
+
+
 # the buffer for the instances lies beside the budget, not in it: 480 KB of it
 # would be missing from the 4 MiB that these frontiers need
 def test_enumeration_buffers_do_not_take_from_the_budget():

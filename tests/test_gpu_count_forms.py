@@ -201,6 +201,62 @@ def test_cliques_of_a_hub_root(d, q):
     assert g.count(q, roots=roots) == g.count(q, roots=roots, warp_granularity=1)
 
 
+def bipartite_with_cliques(d, a, b):
+    """K_{d,d} with a clique of `a` vertices on its left and one of b on its
+    right side; `count(k)` of its k-cliques: any clique of either side (up to
+    one vertex outside the planted ones) with any of the other."""
+    left, right = np.meshgrid(np.arange(d), d + np.arange(d))
+    e = [np.stack([left.ravel(), right.ravel()], 1)]
+    for at, size in ((0, a), (d + 7, b)):
+        x, y = np.triu_indices(size, 1)
+        e.append(np.stack([at + x, at + y], 1))
+    side = lambda size, i: (1, d)[i] if i < 2 else comb(size, i)
+    return csr_of(2 * d, np.concatenate(e)), lambda k: sum(side(a, i) * side(b, k - i) for i in range(k + 1))
+
+
+# every root of a graph whose lists stay long when they are cut to the higher
+# (degree, id): d candidates for each vertex of one side, in every class
+@pytest.mark.parametrize("d", [20, 200, 300, 700, 897, 1000, 1024, 1200])
+@pytest.mark.parametrize("q", [0, 3, 7, 11])
+def test_cliques_of_every_root_with_long_oriented_lists(d, q):
+    csr, count = bipartite_with_cliques(d, 6, 5)
+    g = sme.Graph.from_csr(*csr)
+    g.to_device(0)
+    want = count(sme.query_vertex_count(q))
+    assert want > 0
+    assert g.count(q) == want
+    assert sme.last_stats().paths_processed == g.n  # the matrices counted it
+    o, _ = g.degree_order(orient=True)
+    assert o.count(q, root_stride=1) == want
+
+
+# a budget that has no room for the scratch of the largest class: roots of more
+# than 1024 (6-cliques: 896) candidates go to the level program, and with them
+# a whole task whose lists were cut by (degree, id)
+@pytest.mark.parametrize("n,budget", [(1100, 100), (1100, 300), (1100, 580), (1100, 640), (1024, 300)])
+def test_cliques_without_room_for_the_largest_class(n, budget):
+    g = sme.Graph.clique(n)
+    g.to_device(0)
+    kw = dict(mem_limit_bytes=budget << 20)
+    fits = n <= 1025 or budget >= 640  # twice the scratch's 298 MiB
+    assert g.count(0, **kw) == comb(n, 3)
+    assert (sme.last_stats().paths_processed == n) == fits
+    assert g.count(3, roots=[0, n - 300, 0], **kw) == 2 * comb(n - 1, 3) + comb(299, 3)
+    assert (sme.last_stats().paths_processed == 3) == fits
+
+
+def test_cycles_without_room_for_the_range_queue():
+    # 62 narrow ranges a root: the queue of 100 000 roots takes 50 MB
+    n = 62 * 49152
+    g = sme.Graph.from_csr(*csr_of(n, np.concatenate([random_edges(3000, 20000, 4), [(5, n - 1)]])))
+    g.to_device(0)
+    roots = np.arange(100000, dtype=np.uint32)
+    want = g.count(1, warp_granularity=3)
+    for budget, counters in ((76, False), (400, True)):
+        assert g.count(1, roots=roots, mem_limit_bytes=budget << 20) == want
+        assert (sme.last_stats().paths_processed == len(roots)) == counters
+
+
 @pytest.mark.parametrize("resident", [False, True])
 def test_cliques_of_skewed_graphs(resident):
     g = sme.Graph.rmat(14, 12, seed=2)

@@ -44,7 +44,8 @@ def test_oriented_clique_counts_match_reference(ordered, golden):
             if want is None or want > GPU_LIMIT:
                 continue
             for algo in ALGOS:
-                assert o.count(q, algo) == want, (name, q, algo)
+                for gran in (0, 2):  # 2: the level program's kernel for short lists
+                    assert o.count(q, algo, warp_granularity=gran) == want, (name, q, algo, gran)
             for level in range(4):
                 assert o.count(q, sme.GPU_LIGHT, compress_level=level) == want, (name, q, level)
             assert o.count(q, sme.GPU_GPSM_REUSE, reuse_autogen=1) == want, (name, q)
