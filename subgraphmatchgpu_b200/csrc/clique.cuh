@@ -138,11 +138,16 @@ __global__ void __launch_bounds__(ORI_THREADS) k_orient(const uint64_t* __restri
 constexpr uint32_t kCliqueS = 32, kCliqueM = 256, kCliqueL = 512, kCliqueG = 4096;
 constexpr int kCliqueMThreads = 256;
 constexpr uint32_t CliqueX(int k) { return k == 6 ? 896 : 1024; }
-constexpr int kCliqueParts = 8;      // most parts of a root
-constexpr uint32_t kPartShift = 29;  // queue entries: root index | part << 29
+constexpr int kCliqueParts = 8;  // most CTAs of a root
 
-// Parts a root of d candidates is cut into: its counting work grows faster
-// than the matrix each part builds.
+// CTAs a root of d candidates may occupy: its counting work grows faster than
+// the matrix that each of them builds.  Every root is first taken by one CTA;
+// the others come after all roots have been, claim rows that are not counted
+// yet and find nothing to build where the first one is through (5-cliques, 1500
+// roots of 600 candidates without an edge among them: 1.88 ms with five fixed
+// parts a root, 1.12 by the level program, 0.75 so; every root of R-MAT s18
+// 17.5 ms and 16.8).  Triangles are counted while the rows are found, so there
+// the rows are cut beforehand.
 __device__ __forceinline__ uint32_t CliqueParts(int k, uint32_t d) {
   if (d <= kCliqueM) return 1;
   if (k == 3) return min((uint32_t)kCliqueParts, (d + 127) / 128);
@@ -152,6 +157,7 @@ __device__ __forceinline__ uint32_t CliqueParts(int k, uint32_t d) {
 
 struct CliqueQueues {
   uint32_t* q[5];   // S, M, L, X, G
+  uint32_t* taken;  // rows claimed of each entry of L, then X and G (cleared)
   uint32_t cap[5];
   uint32_t* n;      // entries of each, then the taken ones
   uint32_t* left;   // roots (vertex ids) above every class
@@ -161,8 +167,8 @@ struct CliqueQueues {
   uint32_t* err;
 };
 
-// Sorts the roots into the queues, whose capacities hold every possible entry
-// (one that did not fit would raise the error flag).
+// Sorts the roots (by index) into the queues, whose capacities hold every
+// possible entry (one that did not fit would raise the error flag).
 template <int K, bool ORIENT>
 __global__ void __launch_bounds__(256) k_clique_classify(CView V, const uint32_t* __restrict__ roots, uint32_t P,
                                                          CliqueQueues Q) {
@@ -193,11 +199,9 @@ __global__ void __launch_bounds__(256) k_clique_classify(CView V, const uint32_t
       }
     }
     if (cls >= 2 && cls <= 4) {
-      const uint32_t parts = CliqueParts(K, d);
-      const uint32_t at = atomicAdd(Q.n + cls, parts);
-      for (uint32_t k = 0; k < parts; ++k)
-        if (at + k < Q.cap[cls]) Q.q[cls][at + k] = p | (k << kPartShift);
-        else atomicOr(Q.err, ENGINE_ERR_BOUNDS);
+      const uint32_t at = atomicAdd(Q.n + cls, 1u);
+      if (at < Q.cap[cls]) Q.q[cls][at] = p;
+      else atomicOr(Q.err, ENGINE_ERR_BOUNDS);
     }
     if (cls == 5) {
       const uint32_t at = atomicAdd(Q.nleft, 1u);
@@ -391,6 +395,10 @@ __device__ __forceinline__ uint32_t Expand(const uint32_t* row, uint32_t w0, uin
 constexpr bool CliqueQuads(int k, int threads, bool global) {
   return k >= 5 && threads == kCliqueMThreads && !global;
 }
+// Classes whose roots several CTAs may take.
+constexpr bool CliqueCut(int k, int threads, bool global) {
+  return global || (k != 4 && threads != kCliqueMThreads);
+}
 template <bool QUADS>
 struct RowUnit {
   typedef uint32_t T;
@@ -493,8 +501,8 @@ template <int K, bool ORIENT, int THREADS, bool GLOBAL>
 __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t* __restrict__ roots,
                                                         const uint32_t* __restrict__ q,
                                                         const uint32_t* __restrict__ nq, uint32_t cap,
-                                                        uint32_t* next, uint32_t dmax, uint32_t* scratch,
-                                                        unsigned long long* acc) {
+                                                        uint32_t* next, uint32_t* taken, uint32_t dmax,
+                                                        uint32_t* scratch, unsigned long long* acc) {
   extern __shared__ uint4 cq_sh[];
   constexpr int WARPS = THREADS / 32;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -512,20 +520,25 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
   uint32_t* keys = R + dmax;
   uint16_t* at = reinterpret_cast<uint16_t*>(keys + (1u << tlg));
   uint16_t* lists = (GLOBAL ? reinterpret_cast<uint16_t*>(keys) : at + (1u << tlg)) + (size_t)wid * (K - 3) * dmax;  // K = 3: none
-  __shared__ uint32_t s_item, s_row;
+  __shared__ uint32_t s_more, s_entry, s_part, s_taken, s_row;
+  constexpr bool kParts = CliqueCut(K, THREADS, GLOBAL);
   const uint32_t count = min(*nq, cap);
+  const uint32_t items = count * (kParts ? CliqueParts(K, dmax) : 1);
   unsigned long long local = 0, bytes = 0;
   while (true) {
     if (tid == 0) {
-      s_item = atomicAdd(next, 1u);
+      const uint32_t it = atomicAdd(next, 1u);
+      s_more = it < items;
+      if (it < items) {
+        s_entry = kParts ? it % count : it;
+        s_part = kParts ? it / count : 0;
+        s_taken = kParts && K > 3 && it >= count ? __ldcg(taken + it % count) : 0;
+      }
       s_row = 0;
     }
     __syncthreads();
-    const uint32_t it = s_item;
-    if (it >= count) break;
-    const uint32_t entry = q[it];
-    const uint32_t u0 = __ldg(roots + (entry & ((1u << kPartShift) - 1)));
-    const uint32_t part = entry >> kPartShift;
+    if (!s_more) break;
+    const uint32_t u0 = __ldg(roots + q[s_entry]);
     const uint32_t* L;
     uint32_t d;
     CList<ORIENT>(V, u0, L, d);
@@ -534,7 +547,10 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
       L += r0;
       d -= r0;
     }
-    const uint32_t parts = CliqueParts(K, d);
+    if (kParts && (s_part >= CliqueParts(K, d) || s_taken >= d)) {
+      __syncthreads();  // the item is rewritten
+      continue;
+    }
     const uint32_t W = RowUnits(d, QUADS), ws = W | 1;
     uint32_t* bits_of = reinterpret_cast<uint32_t*>(mat);  // row i's words start at i * ws * kWords
     for (uint32_t i = tid; i < d; i += THREADS) R[i] = __ldg(L + i);
@@ -550,7 +566,7 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
     // one): the lanes fetch the lists of 32 rows at a time, then the warp
     // builds them one by one, four loads in flight per lane (the loads are
     // what a row waits for)
-    const uint32_t row0 = K == 3 ? part : 0, rstep = K == 3 ? parts : 1;
+    const uint32_t row0 = K == 3 && kParts ? s_part : 0, rstep = K == 3 && kParts ? CliqueParts(K, d) : 1;
     const uint32_t nrows = d > row0 ? (d - row0 + rstep - 1) / rstep : 0;
     for (uint32_t i0 = wid; i0 < nrows; i0 += WARPS * 32) {
       const uint32_t mine = i0 + lane * WARPS;
@@ -632,8 +648,8 @@ __global__ void __launch_bounds__(THREADS) k_clique_cta(CView V, const uint32_t*
     __syncthreads();
     while (K > 3) {
       uint32_t i = 0;
-      if (lane == 0) i = atomicAdd(&s_row, 1u);
-      i = __shfl_sync(FULL, i, 0) * parts + part;
+      if (lane == 0) i = atomicAdd(kParts ? taken + s_entry : &s_row, 1u);
+      i = __shfl_sync(FULL, i, 0);
       if (i >= d) break;
       const Unit* row = mat + (size_t)i * ws;
       __syncwarp();

@@ -2476,8 +2476,10 @@ class Executor {
       per_sm = std::max(per_sm, 1);
       if (dv >= 0 && dv < 64) per_sm_of[dv][slot].store(per_sm, std::memory_order_release);
     }
-    const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sms_ * (GLOBAL ? 1 : per_sm), Q.cap[cls]);
-    kernel<<<grid, THREADS, smem, st>>>(V, col, Q.q[cls], Q.n + cls, Q.cap[cls], Q.n + 8 + cls, dmax, scratch,
+    const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sms_ * (GLOBAL ? 1 : per_sm),
+                                                       (uint64_t)Q.cap[cls] * kCliqueParts);
+    uint32_t* taken = Q.taken + (cls > 2 ? Q.cap[2] : 0) + (cls > 3 ? Q.cap[3] : 0);
+    kernel<<<grid, THREADS, smem, st>>>(V, col, Q.q[cls], Q.n + cls, Q.cap[cls], Q.n + 8 + cls, taken, dmax, scratch,
                                          ctrl_);
     Launched();
   }
@@ -2551,24 +2553,23 @@ class Executor {
   // so there one such root sends the whole task to it (false).
   template <int K, bool ORIENT>
   bool CountCliques(const RootTask& task, const uint32_t* col, uint32_t P) {
-    if (P >= (1u << kPartShift)) return false;
+    if (P > 0xFFFFFFFFu / kCliqueParts) return false;
     // entries a class can hold: distinct roots of more than c candidates are
     // at most m / c
-    auto most = [&](uint32_t above, uint32_t parts) {
-      const uint64_t roots = task.list ? P : std::min<uint64_t>(P, g_.m / (above + 1) + 1);
-      return (uint32_t)std::min<uint64_t>(roots * parts, 0xFFFFFFFFull);
+    auto most = [&](uint32_t above) {
+      return (uint32_t)(task.list ? P : std::min<uint64_t>(P, g_.m / (above + 1) + 1));
     };
     // largest possible list: ORIENT keeps neighbours of at least the same
     // degree, so d of them hold d * d of the m stored edges
     const uint64_t bound = ORIENT ? (uint64_t)std::sqrt((double)g_.m) + 1 : g_.n;
     CliqueQueues Q{};
     Q.cap[0] = Q.cap[1] = P;
-    Q.cap[2] = most(kCliqueM, K == 4 ? 1 : 4);
-    Q.cap[3] = most(kCliqueL, K == 4 ? 1 : kCliqueParts);
-    Q.cap[4] = most(CliqueX(K), kCliqueParts);
-    Q.left_cap = most(CliqueX(K), 1);
+    Q.cap[2] = most(kCliqueM);
+    Q.cap[3] = most(kCliqueL);
+    Q.cap[4] = Q.left_cap = most(CliqueX(K));
     const uint64_t tiles = (g_.m + OriTile(g_.m) - 1) / OriTile(g_.m);
-    uint64_t need = 4096 + Q.left_cap * 4ull;
+    const uint64_t ntaken = K == 3 ? 0 : (uint64_t)Q.cap[2] + Q.cap[3] + Q.cap[4];
+    uint64_t need = 4096 + Q.left_cap * 4ull + ntaken * 4;
     for (int c = 0; c < 5; ++c) need += Q.cap[c] * 4ull + 256;
     if (ORIENT) need += g_.n * sizeof(uint2) + (g_.m / 2 + 1) * 4 + tiles * 8 + g_.m / 8 + 2048;
     if (need > A_.Free() / 2) return false;
@@ -2576,6 +2577,10 @@ class Executor {
     uint32_t* ctl = (uint32_t*)A_.Alloc(16 * sizeof(uint32_t));
     for (int c = 0; c < 5; ++c) Q.q[c] = (uint32_t*)A_.Alloc(std::max<size_t>(Q.cap[c], 1) * 4);
     Q.left = (uint32_t*)A_.Alloc(std::max<size_t>(Q.left_cap, 1) * 4);
+    if (ntaken && bound > kCliqueM) {
+      Q.taken = (uint32_t*)A_.Alloc(ntaken * 4);
+      CK(cudaMemsetAsync(Q.taken, 0, ntaken * 4, st_));
+    }
     Q.n = ctl;
     Q.nleft = ctl + 5;
     Q.err = (uint32_t*)(ctrl_ + 3);

@@ -230,6 +230,28 @@ def test_cliques_of_every_root_with_long_oriented_lists(d, q):
     assert o.count(q, root_stride=1) == want
 
 
+def best_ms(g, q, **kw):
+    counts = set()
+    ms = []
+    for _ in range(7):
+        counts.add(g.count(q, **kw))
+        ms.append(sme.last_stats().device_ms)
+    return counts, min(ms)
+
+
+# many roots of 600 candidates without an edge among them: the matrices are all
+# the work, and each is built once
+def test_many_roots_with_empty_neighbourhoods():
+    csr, _ = bipartite_with_cliques(600, 0, 0)
+    g = sme.Graph.from_csr(*csr)
+    g.to_device(0)
+    roots = np.random.default_rng(3).integers(0, g.n, 3000)
+    got, ms = best_ms(g, 7, roots=roots)
+    want, level_ms = best_ms(g, 7, roots=roots, warp_granularity=3)
+    assert got == want == {0}
+    assert ms < 1.2 * level_ms
+
+
 # a budget that has no room for the scratch of the largest class: roots of more
 # than 1024 (6-cliques: 896) candidates go to the level program, and with them
 # a whole task whose lists were cut by (degree, id)
