@@ -155,6 +155,19 @@ __device__ __forceinline__ uint32_t CliqueParts(int k, uint32_t d) {
   return min((uint32_t)kCliqueParts, (d + 127) / 128);
 }
 
+// Roots from which on class X (cls 3) and G are worth their kernels.  One root's
+// matrix keeps a few CTAs busy for milliseconds while the level program spreads
+// it over the device (blocks of R-MAT s18 and s20, matrices and level program):
+// 5-cliques, 1 root of 513-1024 candidates 0.89 and 0.40 ms, 16 roots 1.04 and
+// 1.05; 1 of 2501-4096 100 and 12 ms, 16 100 and 74, 64 153 and 278; 4-cliques,
+// 1 of 1025-1500 0.69 and 0.23, 256 of them 3.0 and 5.8, of 1501-2500 5.7-7.2
+// and 6.0, of 2501-4096 20-25 and 51.  Class X stays where classes M and L keep
+// the device busy for its millisecond anyway (5-cliques of the oriented R-MAT
+// s17 5.0 ms, 5.4 with its few X roots in the level program).
+constexpr uint32_t CliqueLeast(int k, int cls) {
+  return cls == 3 ? (k == 4 ? 1 : 12) : k == 4 ? 128 : 32;
+}
+
 struct CliqueQueues {
   uint32_t* q[5];   // S, M, L, X, G
   uint32_t* taken;  // rows claimed of each entry of L, then X and G (cleared)
@@ -209,6 +222,13 @@ __global__ void __launch_bounds__(256) k_clique_classify(CView V, const uint32_t
       else atomicOr(Q.err, ENGINE_ERR_BOUNDS);
     }
   }
+}
+
+// Roots (vertex ids) of a queue's entries.
+__global__ void k_clique_roots(const uint32_t* __restrict__ roots, const uint32_t* __restrict__ q, uint32_t count,
+                               uint32_t* out) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
+    out[i] = __ldg(roots + q[i]);
 }
 
 // Two lower bounds at once (LowerBound's steps, the loads of both in flight).

@@ -2549,8 +2549,9 @@ class Executor {
   }
 
   // k-cliques over the roots col[0..P) by bit matrices (clique.cuh).  Roots
-  // above every class run the level program; ORIENT has none to hand back,
-  // so there one such root sends the whole task to it (false).
+  // above every class, and few large ones, run the level program; ORIENT has
+  // none to hand back, so there a root above every class sends the whole task
+  // to it (false).
   template <int K, bool ORIENT>
   bool CountCliques(const RootTask& task, const uint32_t* col, uint32_t P) {
     if (P > 0xFFFFFFFFu / kCliqueParts) return false;
@@ -2613,13 +2614,38 @@ class Executor {
     k_clique_classify<K, ORIENT><<<Grid(P, 256), 256, 0, st_>>>(V, col, P, Q);
     Launched();
     TimerStop(to, kPhaseOrganize);
-    uint32_t left = 0;
-    if (bound > Q.top) {  // only then can a root be left
-      left = (uint32_t)ReadU32(Q.nleft);
+    // roots for the level program: those above every class, and those of X and
+    // G where they are few.  Oriented lists have no such program.
+    uint32_t nsteps = 0;
+    uint32_t* steps_roots = nullptr;
+    bool run_x = bound > kCliqueL, run_g = Q.top == kCliqueG;
+    if (ORIENT ? bound > Q.top : bound > (K == 4 ? CliqueX(K) : kCliqueL)) {
+      CK(cudaMemcpyAsync(ctx_.h_pinned, ctl, 6 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st_));
+      CK(cudaStreamSynchronize(st_));
+      const uint32_t* n = reinterpret_cast<const uint32_t*>(ctx_.h_pinned);
+      const uint32_t nx = std::min(n[3], Q.cap[3]), ng = std::min(n[4], Q.cap[4]), left = std::min(n[5], Q.left_cap);
       if (left && ORIENT) {
         A_.Release(mark);
         paths_ -= P;
         return false;
+      }
+      const bool busy = (uint64_t)n[1] + 6ull * n[2] >= 2000;
+      const bool move_x = !ORIENT && !busy && nx < CliqueLeast(K, 3), move_g = !ORIENT && ng < CliqueLeast(K, 4);
+      run_x = run_x && !move_x;
+      run_g = run_g && !move_g;
+      nsteps = left + (move_x ? nx : 0) + (move_g ? ng : 0);
+      if (nsteps) {
+        steps_roots = (uint32_t*)A_.Alloc((size_t)nsteps * 4);
+        uint32_t at = left;
+        if (left) CK(cudaMemcpyAsync(steps_roots, Q.left, (size_t)left * 4, cudaMemcpyDeviceToDevice, st_));
+        auto add = [&](int cls, uint32_t count) {
+          if (!count) return;
+          k_clique_roots<<<Grid(count, 256), 256, 0, st_>>>(col, Q.q[cls], count, steps_roots + at);
+          Launched();
+          at += count;
+        };
+        add(3, move_x ? nx : 0);
+        add(4, move_g ? ng : 0);
       }
     }
     Timed t = TimerStart();
@@ -2631,9 +2657,9 @@ class Executor {
     if (fork) {
       CK(cudaEventRecord(ctx_.copy_ev[0], st_));
       CK(cudaStreamWaitEvent(ctx_.copy_stream, ctx_.copy_ev[0], 0));
-      if (Q.top == kCliqueG)
+      if (run_g)
         LaunchCliqueClass<K, ORIENT, 256, true>(V, col, Q, 4, kCliqueG, scratch, ctx_.copy_stream);
-      if (bound > kCliqueL)
+      if (run_x)
         LaunchCliqueClass<K, ORIENT, kWide, false>(V, col, Q, 3, CliqueX(K), nullptr, ctx_.copy_stream);
       LaunchCliqueClass<K, ORIENT, kWide, false>(V, col, Q, 2, kCliqueL, nullptr, ctx_.copy_stream);
     }
@@ -2645,10 +2671,10 @@ class Executor {
     if (fork) CK(cudaEventRecord(ctx_.copy_ev[1], ctx_.copy_stream));
     if (fork) CK(cudaStreamWaitEvent(st_, ctx_.copy_ev[1], 0));
     TimerStop(t, kPhaseComputeCount);
-    if (left) {
+    if (nsteps) {
       DFront F{};
-      F.P = left;
-      F.inst[(*steps_)[0].u] = Q.left;
+      F.P = nsteps;
+      F.inst[(*steps_)[0].u] = steps_roots;
       Level(1, F);
     }
     A_.Release(mark);

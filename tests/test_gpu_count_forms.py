@@ -157,7 +157,7 @@ def test_few_clique_roots_of_a_large_graph_that_is_not_resident():
     g = sme.Graph.rmat(14, 12, seed=2)
     least = -(-g.m // 6000)
     for count in (least - 1, least):
-        roots = np.arange(count, dtype=np.uint32)
+        roots = np.arange(g.n // 2, g.n // 2 + count, dtype=np.uint32)
         want = g.count(3, roots=roots, warp_granularity=3)
         assert g.count(3, roots=roots) == want
         assert (sme.last_stats().paths_processed == count) == (count == least)
@@ -181,18 +181,39 @@ def test_cliques_of_complete_graphs(n, ks):
         assert g.count(q, roots=[1, 0, 1]) == comb(n - 1, k - 1) + 2 * comb(n - 2, k - 1)
 
 
-# vertex 0 sees every other vertex: a root of d candidates in every class, and
-# above the last one, which keeps the level program
-@pytest.mark.parametrize("d", [31, 256, 257, 700, 896, 897, 960, 961, 1024, 1025, 4096, 4097, 5000])
-@pytest.mark.parametrize("q", [0, 3, 7, 11])
-def test_cliques_of_a_hub_root(d, q):
+def hub_graph(d):
+    """Vertex 0 sees every other of d + 1 vertices, which hold 14 d random
+    edges and a clique of 40."""
     e = np.concatenate([np.stack([np.zeros(d, np.int64), np.arange(1, d + 1)], 1), 1 + random_edges(d, 14 * d, d)])
     rng = np.random.default_rng(d)
     core = rng.choice(np.arange(1, d + 1), min(d, 40), replace=False)
     a, b = np.triu_indices(len(core), 1)
     e = np.concatenate([e, np.stack([core[a], core[b]], 1)])
     rp, cl = csr_of(d + 1, e)
-    g = sme.Graph.from_csr(rp, cl)
+    return sme.Graph.from_csr(rp, cl)
+
+
+# few large roots are left to the level program, which spreads each over the
+# device: class X from 12 on (never for 4-cliques), class G from 32 (128) on
+@pytest.mark.parametrize("d,q,least", [(700, 3, 1), (700, 7, 12), (700, 11, 12), (1500, 3, 128), (1500, 7, 32),
+                                       (1000, 11, 32), (4096, 7, 32)])
+def test_few_large_roots_of_cliques(d, q, least):
+    g = hub_graph(d)
+    g.to_device(0)
+    one = g.count(q, roots=[0], warp_granularity=1)
+    assert one > 0
+    for count in {1, least - 1, least} - {0}:
+        roots = [0] * count + [d]
+        assert g.count(q, roots=roots) == count * one
+        assert (sme.last_stats().paths_processed == len(roots)) == (count >= least)
+
+
+# vertex 0 sees every other vertex: a root of d candidates in every class, and
+# above the last one, which keeps the level program
+@pytest.mark.parametrize("d", [31, 256, 257, 700, 896, 897, 960, 961, 1024, 1025, 4096, 4097, 5000])
+@pytest.mark.parametrize("q", [0, 3, 7, 11])
+def test_cliques_of_a_hub_root(d, q):
+    g = hub_graph(d)
     g.to_device(0)
     want = g.count(q, warp_granularity=1)
     assert want > 0
@@ -263,8 +284,9 @@ def test_cliques_without_room_for_the_largest_class(n, budget):
     fits = n <= 1025 or budget >= 640  # twice the scratch's 298 MiB
     assert g.count(0, **kw) == comb(n, 3)
     assert (sme.last_stats().paths_processed == n) == fits
-    assert g.count(3, roots=[0, n - 300, 0], **kw) == 2 * comb(n - 1, 3) + comb(299, 3)
-    assert (sme.last_stats().paths_processed == 3) == fits
+    roots = [0] * 130 + [n - 300]  # enough for the largest class
+    assert g.count(3, roots=roots, **kw) == 130 * comb(n - 1, 3) + comb(299, 3)
+    assert (sme.last_stats().paths_processed == len(roots)) == fits
 
 
 def test_cycles_without_room_for_the_range_queue():
