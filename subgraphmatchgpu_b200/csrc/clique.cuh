@@ -155,17 +155,18 @@ __device__ __forceinline__ uint32_t CliqueParts(int k, uint32_t d) {
   return min((uint32_t)kCliqueParts, (d + 127) / 128);
 }
 
-// Roots from which on class X (cls 3) and G are worth their kernels.  One root's
+// Roots from which on classes L (cls 2), X and G are worth their kernels.  One root's
 // matrix keeps a few CTAs busy for milliseconds while the level program spreads
 // it over the device (blocks of R-MAT s18 and s20, matrices and level program):
 // 5-cliques, 1 root of 513-1024 candidates 0.89 and 0.40 ms, 16 roots 1.04 and
 // 1.05; 1 of 2501-4096 100 and 12 ms, 16 100 and 74, 64 153 and 278; 4-cliques,
 // 1 of 1025-1500 0.69 and 0.23, 256 of them 3.0 and 5.8, of 1501-2500 5.7-7.2
-// and 6.0, of 2501-4096 20-25 and 51.  Class X stays where classes M and L keep
-// the device busy for its millisecond anyway (5-cliques of the oriented R-MAT
+// and 6.0, of 2501-4096 20-25 and 51; 6-cliques, 1 of 257-512 5.1 and 1.3, 16
+// 5.1 and 2.8, 16 of 513-1024 11.4 and 9.0.  Classes L and X stay where classes M and L keep
+// the device busy for as long anyway (5-cliques of the oriented R-MAT
 // s17 5.0 ms, 5.4 with its few X roots in the level program).
 constexpr uint32_t CliqueLeast(int k, int cls) {
-  return cls == 3 ? (k == 4 ? 1 : 12) : k == 4 ? 128 : 32;
+  return k == 4 ? (cls == 4 ? 128 : 1) : cls == 4 ? 32 : k == 5 ? (cls == 3 ? 12 : 1) : (cls == 3 ? 32 : 48);
 }
 
 struct CliqueQueues {

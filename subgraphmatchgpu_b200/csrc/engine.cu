@@ -20,6 +20,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstdio>
+#include <cstring>
 #include <string>
 
 #include "clique.cuh"
@@ -2614,38 +2615,40 @@ class Executor {
     k_clique_classify<K, ORIENT><<<Grid(P, 256), 256, 0, st_>>>(V, col, P, Q);
     Launched();
     TimerStop(to, kPhaseOrganize);
-    // roots for the level program: those above every class, and those of X and
-    // G where they are few.  Oriented lists have no such program.
+    // roots for the level program: those above every class, and those of L, X
+    // and G where they are few.  Oriented lists have no such program.
     uint32_t nsteps = 0;
     uint32_t* steps_roots = nullptr;
-    bool run_x = bound > kCliqueL, run_g = Q.top == kCliqueG;
-    if (ORIENT ? bound > Q.top : bound > (K == 4 ? CliqueX(K) : kCliqueL)) {
+    bool run[5] = {true, true, true, bound > kCliqueL, Q.top == kCliqueG};
+    if (ORIENT ? bound > Q.top : bound > (K == 4 ? CliqueX(K) : K == 5 ? kCliqueL : kCliqueM)) {
       CK(cudaMemcpyAsync(ctx_.h_pinned, ctl, 6 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st_));
       CK(cudaStreamSynchronize(st_));
-      const uint32_t* n = reinterpret_cast<const uint32_t*>(ctx_.h_pinned);
-      const uint32_t nx = std::min(n[3], Q.cap[3]), ng = std::min(n[4], Q.cap[4]), left = std::min(n[5], Q.left_cap);
+      uint32_t n[5];
+      std::memcpy(n, ctx_.h_pinned, sizeof(n));
+      for (int c = 0; c < 5; ++c) n[c] = std::min(n[c], Q.cap[c]);
+      const uint32_t left = std::min(reinterpret_cast<const uint32_t*>(ctx_.h_pinned)[5], Q.left_cap);
       if (left && ORIENT) {
         A_.Release(mark);
         paths_ -= P;
         return false;
       }
-      const bool busy = (uint64_t)n[1] + 6ull * n[2] >= 2000;
-      const bool move_x = !ORIENT && !busy && nx < CliqueLeast(K, 3), move_g = !ORIENT && ng < CliqueLeast(K, 4);
-      run_x = run_x && !move_x;
-      run_g = run_g && !move_g;
-      nsteps = left + (move_x ? nx : 0) + (move_g ? ng : 0);
+      const bool busy = (uint64_t)n[1] + 6ull * n[2] >= (K == 6 ? 8000 : 2000);
+      nsteps = left;
+      for (int c = 2; c < 5; ++c)
+        if (!ORIENT && n[c] < CliqueLeast(K, c) && (c == 4 || !busy)) {
+          run[c] = false;
+          nsteps += n[c];
+        }
       if (nsteps) {
         steps_roots = (uint32_t*)A_.Alloc((size_t)nsteps * 4);
-        uint32_t at = left;
         if (left) CK(cudaMemcpyAsync(steps_roots, Q.left, (size_t)left * 4, cudaMemcpyDeviceToDevice, st_));
-        auto add = [&](int cls, uint32_t count) {
-          if (!count) return;
-          k_clique_roots<<<Grid(count, 256), 256, 0, st_>>>(col, Q.q[cls], count, steps_roots + at);
+        uint32_t at = left;
+        for (int c = 2; c < 5; ++c) {
+          if (run[c] || !n[c]) continue;
+          k_clique_roots<<<1, 256, 0, st_>>>(col, Q.q[c], n[c], steps_roots + at);
           Launched();
-          at += count;
-        };
-        add(3, move_x ? nx : 0);
-        add(4, move_g ? ng : 0);
+          at += n[c];
+        }
       }
     }
     Timed t = TimerStart();
@@ -2657,11 +2660,12 @@ class Executor {
     if (fork) {
       CK(cudaEventRecord(ctx_.copy_ev[0], st_));
       CK(cudaStreamWaitEvent(ctx_.copy_stream, ctx_.copy_ev[0], 0));
-      if (run_g)
+      if (run[4])
         LaunchCliqueClass<K, ORIENT, 256, true>(V, col, Q, 4, kCliqueG, scratch, ctx_.copy_stream);
-      if (run_x)
+      if (run[3])
         LaunchCliqueClass<K, ORIENT, kWide, false>(V, col, Q, 3, CliqueX(K), nullptr, ctx_.copy_stream);
-      LaunchCliqueClass<K, ORIENT, kWide, false>(V, col, Q, 2, kCliqueL, nullptr, ctx_.copy_stream);
+      if (run[2])
+        LaunchCliqueClass<K, ORIENT, kWide, false>(V, col, Q, 2, kCliqueL, nullptr, ctx_.copy_stream);
     }
     if (bound > kCliqueS)
       LaunchCliqueClass<K, ORIENT, kCliqueMThreads, false>(V, col, Q, 1, kCliqueM, nullptr, st_);

@@ -194,9 +194,10 @@ def hub_graph(d):
 
 
 # few large roots are left to the level program, which spreads each over the
-# device: class X from 12 on (never for 4-cliques), class G from 32 (128) on
-@pytest.mark.parametrize("d,q,least", [(700, 3, 1), (700, 7, 12), (700, 11, 12), (1500, 3, 128), (1500, 7, 32),
-                                       (1000, 11, 32), (4096, 7, 32)])
+# device: class L of 6-cliques from 48 on, class X from 12 (32 for 6-cliques, 1
+# for 4-cliques), class G from 32 (128) on
+@pytest.mark.parametrize("d,q,least", [(400, 3, 1), (400, 7, 1), (400, 11, 48), (700, 3, 1), (700, 7, 12), (700, 11, 32),
+                                       (1500, 3, 128), (1500, 7, 32), (1000, 11, 32), (4096, 7, 32)])
 def test_few_large_roots_of_cliques(d, q, least):
     g = hub_graph(d)
     g.to_device(0)
