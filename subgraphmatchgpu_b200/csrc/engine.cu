@@ -2255,6 +2255,7 @@ class Executor {
       : prog_(prog), g_(g), ctx_(ctx), A_(ctx.arena), st_(ctx.stream), out_(d_out), cap_(cap), steps_(&prog.steps) {
     sms_ = SmCount(ctx.device);
     mat_misses_.assign(std::max(prog.steps.size(), prog.minus.size()), 0);
+    mat_skips_ = mat_misses_;
     lists_simple_ = g.defects >= 0 && !((uint32_t)g.defects & kNotSimple);
   }
 
@@ -2390,8 +2391,8 @@ class Executor {
   double ext_overlap_ = 32.0;
   int ext_misses_ = 0;  // counting frontiers whose lists did not fit at once
   // per step: frontiers whose children did not fit the budget at once, less
-  // those whose children did
-  std::vector<int> mat_misses_;
+  // three times those whose children did
+  std::vector<int> mat_misses_, mat_skips_;
 
   // The steps over the roots left_[0..n).
   void RunLeft(uint32_t n) {
@@ -3408,12 +3409,14 @@ class Executor {
     } else if (s.kind == S_MATERIALIZE) {
       // one batch when all children fit, counted exactly; else batches by the
       // set sizes, an upper bound, each counted in its turn.  A step that
-      // misses more often than it fits is not tried again: under a small budget
-      // its frontiers would all be counted twice (R-MAT s14, diamonds under 4
-      // MiB by the reuse plan: 6.5 ms without tries, 7.6 with one per frontier,
-      // 6.5 so; 5-cliques under 8 MiB by GPSM, which fit: 35, 22 and 22 ms).
+      // misses three times as often as it fits tries one frontier in eight:
+      // under a small budget its frontiers would all be counted twice (R-MAT
+      // s14, diamonds under 4 MiB by the reuse plan: 6.5 ms without tries, 7.6
+      // with one per frontier, 6.7 so; 5-cliques under 8 MiB by GPSM, which fit:
+      // 35, 22 and 22 ms; 4-cliques of R-MAT s16, external, 13 MiB: 189 ms with
+      // one per frontier, 205 where three misses end the tries, 183 so).
       const double pf = 16, cf = 4.0 * (s.mat_after.size() + s.sets_after.size()) + 16;
-      if (mat_misses_[k] < 3) {
+      if (mat_misses_[k] < 3 || ++mat_skips_[k] % 8 == 0) {
         Timed to = TimerStart();
         uint64_t* cnt = (uint64_t*)A_.Alloc((size_t)F.P * 8);
         uint32_t* first = FirstOf(dc, F.P);
@@ -3421,12 +3424,12 @@ class Executor {
         TimerStop(to, kPhaseOrganize);
         if (pf * F.P + cf * (double)t.est <= (double)Budget(k) && t.est <= 2000000000ull) {
           ++batches_;
-          mat_misses_[k] = std::max(mat_misses_[k] - 1, -8);
+          mat_misses_[k] = std::max(mat_misses_[k] - 3, -8);
           Materialize(k, F, dc, cnt, first, t.est);
           A_.Release(mark0);
           return;
         }
-        ++mat_misses_[k];
+        mat_misses_[k] = std::min(mat_misses_[k] + 1, 3);
         A_.Release(mark0);
       }
       est = (uint64_t*)A_.Alloc((size_t)F.P * 8);
