@@ -11,12 +11,13 @@
 // only as a task of every root (see ORIENT).  Nothing is
 // materialised and nothing leaves the SM but the count.  Whole
 // calls, level program against this: 4-cliques of R-MAT s18 ef16, every root
-// 73.0 -> 2.2 ms; 5-cliques of the oriented R-MAT s17 ef16 187 -> 5.6 ms;
-// 4-cliques of 16 384 roots of R-MAT s20 ef16 0.91 -> 0.40 ms.
+// 73.0 -> 2.1 ms; 5-cliques of the oriented R-MAT s17 ef16 187 -> 5.0 ms;
+// 4-cliques of 16 384 roots of R-MAT s20 ef16 0.91 -> 0.31 ms.
 //
 // Few roots are bound by the latency of the build's loads (hub bitmap words
 // from HBM): hence four of them in flight per lane, 32 lists fetched at once
-// and many warps per root (4-cliques, s20 roots: 0.80 -> 0.40 ms).  Many roots
+// and many warps per root (4-cliques, s20 roots: 0.80 -> 0.40 ms; 0.31 with the
+// small class beside class M).  Many roots
 // are bound by instruction issue: hence the candidates' hash table (1-2
 // shared-memory reads per looked-up element, a binary search takes 8), the
 // member lists compacted from their parent's by ballot (5-cliques, s17: 18 ->
@@ -26,12 +27,13 @@
 // A root's cost grows with d, so roots are sorted into classes by d: up to 32
 // a warp and one word per row (k_clique_small); up to 256, 512 and 1024 (896
 // for k = 6) a CTA with the matrix in shared memory; up to 4096 a CTA with
-// the matrix in global scratch.  A large root's rows are cut into parts that
-// different CTAs take, each with a matrix of its own.
+// the matrix in global scratch.  CTAs that find no root left help with the rows
+// of large ones, each with a matrix of its own (CliqueParts); where large roots
+// are few the level program takes them (CliqueLeast).
 //
 // ORIENT: the task is every root of a symmetric graph, whose count does not
 // depend on the order of the vertices; the lists are then cut to the
-// neighbours of higher (degree, id) first (k_orient_*), which bounds d by the
+// neighbours of higher (degree, id) first (k_orient), which bounds d by the
 // square root of the stored edges (on R-MAT s18 the largest list falls from 15
 // thousand to a few hundred).  The lists stay sorted by id, the matrix by
 // index.

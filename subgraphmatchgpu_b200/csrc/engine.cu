@@ -141,9 +141,9 @@ __device__ __forceinline__ uint64_t EstOf(const DFront& F, const DStep& s, const
 // sums into exclusive ones with the total after them.  One tile needs nothing
 // more; k_scan_add adds the tile sums otherwise.  The estimate, its scan and
 // the total were four launches and the host's split query before.  ITEMS 1
-// for frontiers of up to kScanSmall paths (an estimate is a chain of loads:
+// for frontiers of up to kScanSmall paths an SM (an estimate is a chain of loads:
 // one per thread, over as many SMs as there are tiles), else SCAN_ITEMS.
-constexpr uint32_t kScanSmall = 148 * 4 * SCAN_THREADS;
+constexpr uint32_t kScanSmall = 4 * SCAN_THREADS;
 template <EstKind KIND, bool TWO, int ITEMS>
 __global__ void __launch_bounds__(SCAN_THREADS) k_est_scan(DFront F, DStep s, DCond c,
                                                            const uintE* __restrict__ rp, uint64_t* out,
@@ -1679,6 +1679,17 @@ int DeviceCount() {
   return n;
 }
 
+namespace {
+int SmCount(int device) {
+  static int cached[64] = {0};
+  if (device >= 0 && device < 64 && cached[device]) return cached[device];
+  int v = 148;
+  cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device);
+  if (device >= 0 && device < 64) cached[device] = v;
+  return v;
+}
+}  // namespace
+
 DeviceContext::~DeviceContext() {}
 
 DeviceContext* CreateContext(int device, uint64_t bytes) {
@@ -2082,7 +2093,8 @@ void LaunchCheck(const DeviceGraph& g, bool sym, uint32_t* flag, cudaStream_t st
   if (!g.m) return;
   // a chunk is a serial chain for its warp: short ones while there are few
   const uint32_t chunk = g.m < (4u << 20) ? 64 : 512;
-  const unsigned grid = (unsigned)std::min<uint64_t>((g.m + (uint64_t)chunk * 8 - 1) / ((uint64_t)chunk * 8), 148 * 8);
+  const unsigned grid = (unsigned)std::min<uint64_t>((g.m + (uint64_t)chunk * 8 - 1) / ((uint64_t)chunk * 8),
+                                                     (uint64_t)SmCount(g.device) * 8);
   if (sym)
     k_check_simple<true><<<grid, WARP_BLOCK, 0, st>>>(ViewOf(g), (uint32_t)g.n, g.m, chunk, flag);
   else
@@ -2208,15 +2220,6 @@ void FreeDeviceGraph(DeviceGraph* d) {
 
 // --------------------------------------------------------------- executor --
 namespace {
-
-int SmCount(int device) {
-  static int cached[64] = {0};
-  if (device >= 0 && device < 64 && cached[device]) return cached[device];
-  int v = 148;
-  cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device);
-  if (device >= 0 && device < 64) cached[device] = v;
-  return v;
-}
 
 DCond ToDCond(const std::vector<StepCond>& c) {
   DCond d{};
@@ -3167,7 +3170,7 @@ class Executor {
   template <EstKind KIND>
   Totals EstScan(const DFront& F, const DStep& ds, const DCond& dc, uint64_t* est, uint64_t* est2,
                  uint32_t* first = nullptr, bool read = true) {
-    const uint32_t tile = F.P <= kScanSmall ? SCAN_THREADS : SCAN_TILE;
+    const uint32_t tile = F.P <= kScanSmall * (uint32_t)sms_ ? SCAN_THREADS : SCAN_TILE;
     const uint32_t nb = (F.P + tile - 1) / tile;
     const size_t m = A_.Mark();
     uint64_t* bs = (uint64_t*)A_.Alloc(((size_t)nb + 1) * 16);
