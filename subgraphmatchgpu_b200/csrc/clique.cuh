@@ -171,11 +171,25 @@ constexpr uint32_t CliqueLeast(int k, int cls) {
   return k == 4 ? (cls == 4 ? 128 : 1) : cls == 4 ? 32 : k == 5 ? (cls == 3 ? 12 : 1) : (cls == 3 ? 32 : 48);
 }
 
+// Whether class G pays by how many of kCliqueSamples sampled pairs a root are
+// joined: the matrix costs a look-up per list element whatever it holds, the
+// level program ends where nothing is joined.  1000 roots with the same 1400 or
+// 3000 candidates, matrices and level program, 4-cliques: no pair joined 3.1
+// and 0.8, 11.9 and 1.6 ms, 1% 4.4 and 4.3, 19.1 and 17.5, 5% 5.6 and 18.6,
+// 31.2 and 91.3; 5-cliques, 128 roots: 1% 1.1 and 0.8, 5.6 and 3.2, 5% 4.2 and
+// 5.8, 43.5 and 38.8, 10% 11.9 and 24.2, 143 and 208; where the joined pairs are
+// clustered the matrices win from fewer on (R-MAT s18, 256 roots of 1025-1500,
+// between 3 and 6%: 17.7 and 90.8).
+constexpr uint32_t kCliqueSamples = 4;
+constexpr bool CliqueDense(int k, uint64_t joined, uint64_t roots) {
+  return joined * 100 >= (k == 4 ? 2 : 3) * kCliqueSamples * roots;
+}
+
 struct CliqueQueues {
   uint32_t* q[5];   // S, M, L, X, G
   uint32_t* taken;  // rows claimed of each entry of L, then X and G (cleared)
   uint32_t cap[5];
-  uint32_t* n;      // entries of each, then the taken ones
+  uint32_t* n;      // entries of each, left roots, joined pairs of G's samples, then the taken entries
   uint32_t* left;   // roots (vertex ids) above every class
   uint32_t left_cap;
   uint32_t* nleft;
@@ -193,11 +207,15 @@ __global__ void __launch_bounds__(256) k_clique_classify(CView V, const uint32_t
   for (uint32_t base = w0; base < P; base += gridDim.x * blockDim.x) {
     const uint32_t p = base + lane;
     uint32_t d = 0, u0 = 0;
+    const uint32_t* a = nullptr;
     if (p < P) {
       u0 = __ldg(roots + p);
-      const uint32_t* a;
       CList<ORIENT>(V, u0, a, d);
-      if (!ORIENT) d -= LowerBound(a, d, u0 + 1);
+      if (!ORIENT) {
+        const uint32_t r0 = LowerBound(a, d, u0 + 1);
+        a += r0;
+        d -= r0;
+      }
     }
     int cls = -1;
     if (d >= K - 1)
@@ -218,6 +236,25 @@ __global__ void __launch_bounds__(256) k_clique_classify(CView V, const uint32_t
       const uint32_t at = atomicAdd(Q.n + cls, 1u);
       if (at < Q.cap[cls]) Q.q[cls][at] = p;
       else atomicOr(Q.err, ENGINE_ERR_BOUNDS);
+    }
+    if (!ORIENT && cls == 4) {  // d is above a thousand
+      uint32_t joined = 0;
+      for (uint32_t t = 1; t <= kCliqueSamples; ++t) {
+        const uint32_t h = (p * kCliqueSamples + t) * 2654435761u;
+        const uint32_t i = (h >> 16) % d, k = (i + 1 + (h & 0xFFFFu) % (d - 1)) % d;  // k != i
+        const uint32_t x = __ldg(a + min(i, k)), y = __ldg(a + max(i, k));
+        const uint32_t* bm = HubBitmap(V.G, x);
+        if (bm) {
+          joined += BitTest(bm, y);
+        } else {
+          const uint32_t* b;
+          uint32_t len;
+          AdjList(V.G, x, b, len);
+          const uint32_t pos = LowerBound(b, len, y);
+          joined += pos < len && __ldg(b + pos) == y;
+        }
+      }
+      if (joined) atomicAdd(Q.n + 6, joined);
     }
     if (cls == 5) {
       const uint32_t at = atomicAdd(Q.nleft, 1u);

@@ -2620,17 +2620,19 @@ class Executor {
     Launched();
     TimerStop(to, kPhaseOrganize);
     // roots for the level program: those above every class, and those of L, X
-    // and G where they are few.  Oriented lists have no such program.
+    // and G where they are few (of G also where their candidates are hardly
+    // joined).  Oriented lists have no such program.
     uint32_t nsteps = 0;
     uint32_t* steps_roots = nullptr;
     bool run[5] = {true, true, true, bound > kCliqueL, Q.top == kCliqueG};
     if (ORIENT ? bound > Q.top : bound > (K == 4 ? CliqueX(K) : K == 5 ? kCliqueL : kCliqueM)) {
-      CK(cudaMemcpyAsync(ctx_.h_pinned, ctl, 6 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st_));
+      CK(cudaMemcpyAsync(ctx_.h_pinned, ctl, 7 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st_));
       CK(cudaStreamSynchronize(st_));
       uint32_t n[5];
       std::memcpy(n, ctx_.h_pinned, sizeof(n));
       for (int c = 0; c < 5; ++c) n[c] = std::min(n[c], Q.cap[c]);
       const uint32_t left = std::min(reinterpret_cast<const uint32_t*>(ctx_.h_pinned)[5], Q.left_cap);
+      const uint32_t joined = reinterpret_cast<const uint32_t*>(ctx_.h_pinned)[6];
       if (left && ORIENT) {
         A_.Release(mark);
         paths_ -= P;
@@ -2639,7 +2641,8 @@ class Executor {
       const bool busy = (uint64_t)n[1] + 6ull * n[2] >= (K == 6 ? 8000 : 2000);
       nsteps = left;
       for (int c = 2; c < 5; ++c)
-        if (!ORIENT && n[c] < CliqueLeast(K, c) && (c == 4 || !busy)) {
+        if (!ORIENT && (c == 4 ? n[c] < CliqueLeast(K, c) || !CliqueDense(K, joined, n[c])
+                               : n[c] < CliqueLeast(K, c) && !busy)) {
           run[c] = false;
           nsteps += n[c];
         }
@@ -2649,7 +2652,7 @@ class Executor {
         uint32_t at = left;
         for (int c = 2; c < 5; ++c) {
           if (run[c] || !n[c]) continue;
-          k_clique_roots<<<1, 256, 0, st_>>>(col, Q.q[c], n[c], steps_roots + at);
+          k_clique_roots<<<Grid(n[c], 256), 256, 0, st_>>>(col, Q.q[c], n[c], steps_roots + at);
           Launched();
           at += n[c];
         }

@@ -181,10 +181,10 @@ def test_cliques_of_complete_graphs(n, ks):
         assert g.count(q, roots=[1, 0, 1]) == comb(n - 1, k - 1) + 2 * comb(n - 2, k - 1)
 
 
-def hub_graph(d):
-    """Vertex 0 sees every other of d + 1 vertices, which hold 14 d random
+def hub_graph(d, each=14):
+    """Vertex 0 sees every other of d + 1 vertices, which hold `each` d random
     edges and a clique of 40."""
-    e = np.concatenate([np.stack([np.zeros(d, np.int64), np.arange(1, d + 1)], 1), 1 + random_edges(d, 14 * d, d)])
+    e = np.concatenate([np.stack([np.zeros(d, np.int64), np.arange(1, d + 1)], 1), 1 + random_edges(d, each * d, d)])
     rng = np.random.default_rng(d)
     core = rng.choice(np.arange(1, d + 1), min(d, 40), replace=False)
     a, b = np.triu_indices(len(core), 1)
@@ -197,9 +197,9 @@ def hub_graph(d):
 # device: class L of 6-cliques from 48 on, class X from 12 (32 for 6-cliques, 1
 # for 4-cliques), class G from 32 (128) on
 @pytest.mark.parametrize("d,q,least", [(400, 3, 1), (400, 7, 1), (400, 11, 48), (700, 3, 1), (700, 7, 12), (700, 11, 32),
-                                       (1500, 3, 128), (1500, 7, 32), (1000, 11, 32), (4096, 7, 32)])
+                                       (1500, 3, 128), (1500, 7, 32), (1000, 11, 32), (4096, 3, 128)])
 def test_few_large_roots_of_cliques(d, q, least):
-    g = hub_graph(d)
+    g = hub_graph(d, 14 if d < 1000 else d // 10)  # class G: a fifth of the pairs joined
     g.to_device(0)
     one = g.count(q, roots=[0], warp_granularity=1)
     assert one > 0
@@ -207,6 +207,23 @@ def test_few_large_roots_of_cliques(d, q, least):
         roots = [0] * count + [d]
         assert g.count(q, roots=roots) == count * one
         assert (sme.last_stats().paths_processed == len(roots)) == (count >= least)
+
+
+# roots of class G whose candidates are hardly joined, or joined well: the
+# level program ends early on the former, the matrices do not
+@pytest.mark.parametrize("joined,matrices", [(0.0, False), (0.005, False), (0.12, True)])
+@pytest.mark.parametrize("q", [3, 7])
+def test_large_roots_by_how_their_candidates_are_joined(q, joined, matrices):
+    hubs, d = 200, 1200
+    x, y = np.meshgrid(np.arange(hubs), hubs + np.arange(d))
+    e = np.concatenate([np.stack([x.ravel(), y.ravel()], 1),
+                        hubs + random_edges(d, int(joined * d * d / 2) + 2, 5)])
+    g = sme.Graph.from_csr(*csr_of(hubs + d, e))
+    g.to_device(0)
+    roots = np.arange(hubs)
+    assert g.count(q, roots=roots) == g.count(q, roots=roots[:1], warp_granularity=3) * hubs
+    g.count(q, roots=roots)
+    assert (sme.last_stats().paths_processed == hubs) == matrices
 
 
 # vertex 0 sees every other vertex: a root of d candidates in every class, and
